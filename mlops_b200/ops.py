@@ -414,23 +414,29 @@ def dswiglu_routed(h13, r, route_weights, order, *, limit=None, quantized=True, 
 
 
 @_on_tensor_device
-def quantize_blocks(weight):
+def quantize_blocks(weight, *, out=None):
     """(data E4M3 [E,out,in], scale fp32 [E, ceil(out/128), ceil(in/128)]) of a bf16 or
-    fp32 weight."""
-    _need_cuda(weight)
+    fp32 weight, written into `out = (data, scale)` when given (contiguous, not overlapping
+    `weight`)."""
+    _need_cuda(weight, *(out or ()))
     if weight.dim() != 3:
         raise NativeError("Expected an [experts, out, in] weight")
     weight = weight.contiguous()
     if weight.dtype not in (torch.bfloat16, torch.float32):
         weight = weight.float()
-    experts, out, inner = weight.shape
-    data = torch.empty(weight.shape, dtype=FP8, device=weight.device)
-    scale = torch.empty(
-        (experts, (out + 127) // 128, (inner + 127) // 128), dtype=torch.float32, device=weight.device
-    )
+    experts, rows, inner = weight.shape
+    scale_shape = (experts, (rows + 127) // 128, (inner + 127) // 128)
+    if out is None:
+        data = torch.empty(weight.shape, dtype=FP8, device=weight.device)
+        scale = torch.empty(scale_shape, dtype=torch.float32, device=weight.device)
+    else:
+        data, scale = out
+        if (data.shape != weight.shape or data.dtype != FP8 or tuple(scale.shape) != scale_shape
+                or scale.dtype != torch.float32 or not data.is_contiguous() or not scale.is_contiguous()):
+            raise NativeError("out must be contiguous E4M3 data and fp32 scales of the weight's shape")
     check(
         lib.b200moe_quantize_blocks(
-            weight.data_ptr(), 1 if weight.dtype == torch.float32 else 0, experts, out, inner,
+            weight.data_ptr(), 1 if weight.dtype == torch.float32 else 0, experts, rows, inner,
             data.data_ptr(), scale.data_ptr(), _stream(),
         ),
         "quantize_blocks",

@@ -80,6 +80,16 @@ def _clone(func, args, kwargs):
     return BlockFP8Weight(source._data.clone(), source._scale.clone(), dtype=source.dtype)
 
 
+def _quantises_in_place(target, source) -> bool:
+    """Whether the quantiser may write `source`'s blocks straight into `target`'s buffers: equal
+    shapes, dense buffers, and a source that does not share their memory (the quantiser reads it
+    while it writes). Anything else is quantised into fresh tensors and copied."""
+    buffers = (target._data, target._scale)
+    return (type(source) in (torch.Tensor, torch.nn.Parameter) and source.shape == target._data.shape
+            and all(b.is_contiguous() and b.device == source.device and not b.is_inference()
+                    and b.untyped_storage().data_ptr() != source.untyped_storage().data_ptr() for b in buffers))
+
+
 def _copy(func, args, kwargs):
     target, source = args[0], args[1]
     if not isinstance(target, BlockFP8Weight):  # container -> ordinary tensor: its values
@@ -87,7 +97,12 @@ def _copy(func, args, kwargs):
     if isinstance(source, BlockFP8Weight):
         data, scale = source._data, source._scale
     else:  # publication of a master weight: quantise it as at construction
-        data, scale = ops.quantize_blocks(source.to(target.device))
+        source = source.to(target.device)
+        if _quantises_in_place(target, source):
+            ops.quantize_blocks(source, out=(target._data, target._scale))
+            torch.autograd.graph.increment_version((target._data, target._scale))  # written behind autograd's back
+            return target
+        data, scale = ops.quantize_blocks(source)
     target._data.copy_(data)
     target._scale.copy_(scale)
     return target

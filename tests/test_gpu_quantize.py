@@ -28,6 +28,58 @@ def test_weight_blocks_match_reference_fixture(golden):
         assert torch.equal(scale.cpu(), fixture[name + "_scale"])
 
 
+@pytest.mark.parametrize("shape", [(1, 128, 128), (2, 8, 8), (3, 200, 328), (1, 129, 4), (2, 64, 1000)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("special", [False, True])
+def test_weight_blocks_of_aligned_and_unaligned_sources(shape, dtype, special):
+    """The one-pass quantiser (16-byte loads) writes the bytes and scales of the value-by-value one,
+    which serves a source one element off alignment; both equal the oracle where it is defined by
+    finite values. Infinities and NaN: the maximum skips a NaN, an infinity makes the scale
+    infinite, and a NaN quotient is stored as -448."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(sum(shape))
+    n = shape[0] * shape[1] * shape[2]
+    w = (torch.randn(n, generator=g) * torch.rand(n, generator=g).mul(40).sub(20).exp2()).to(dtype).view(shape)
+    if special:
+        w.view(-1)[3] = float("nan")
+        w[-1, -1, -1] = float("-inf")
+    else:
+        w[0, 0, :4] = 0
+    store = torch.empty(n + 1, dtype=dtype, device=DEV)
+    store[1:] = w.to(DEV).view(-1)
+    q, s = ops.quantize_blocks(w.to(DEV))
+    q_general, s_general = ops.quantize_blocks(store[1:].view(shape))
+    assert torch.equal(q.view(U8), q_general.view(U8))
+    assert torch.equal(s, s_general)
+    if not special:
+        q_ref, s_ref = O.quantize_blocks(w)
+        assert torch.equal(q.cpu().view(U8), q_ref.view(U8)) and torch.equal(s.cpu(), s_ref)
+
+
+def test_publication_writes_the_container_in_place():
+    """`container.copy_(master)` fills the container's own buffers, a master that shares their
+    memory or broadcasts included, and tells autograd that they changed."""
+    from mlops_b200.weights import BlockFP8Weight
+
+    ops = _ops()
+    g = torch.Generator().manual_seed(5)
+    master = torch.randn(3, 256, 128, generator=g).to(DEV)
+    ref, ref_scale = ops.quantize_blocks(master)
+    container = BlockFP8Weight(torch.zeros_like(ref), torch.zeros_like(ref_scale))
+    data, scale, versions = container._data, container._scale, (container._data._version, container._scale._version)
+    container.copy_(master)
+    assert container._data is data and container._scale is scale
+    assert torch.equal(data.view(U8), ref.view(U8)) and torch.equal(scale, ref_scale)
+    assert data._version > versions[0] and scale._version > versions[1]
+    container.copy_(master[:1])  # broadcast over the experts
+    assert torch.equal(data.view(U8), ref[:1].expand_as(ref).view(U8))
+    store = torch.empty(master.numel(), device=DEV)  # the master's memory holds the container's bytes
+    shared = BlockFP8Weight(store.view(torch.float8_e4m3fn)[:master.numel()].view(3, 256, 128), torch.zeros_like(scale))
+    store.view(3, 256, 128).copy_(master)
+    shared.copy_(store.view(3, 256, 128))
+    assert torch.equal(shared._data.view(U8), ref.view(U8))
+
+
 def test_row_quantiser_matches_reference_fixture(golden):
     ops = _ops()
     fixture = golden("quantize.pt")
