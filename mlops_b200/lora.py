@@ -304,6 +304,7 @@ def _setup_context(ctx, inputs, output):
     ctx.weight_grad_dtype = provider._context_weight_gradient_dtype()
     ctx.logical = gate_up.dtype if gate_up.dtype != torch.float8_e4m3fn else torch.bfloat16
     ctx.mark_non_differentiable(counts, logits, weights, ids, order, offsets, slots, h13, t1, t2)
+    ctx.set_materialize_grads(False)  # no zeros for the residual outputs (h13 alone is [rows, 2F])
 
 
 def _autograd_backward(ctx, grad_output, grad_aux, _g_counts, grad_probability_sum, *_metadata_grads):

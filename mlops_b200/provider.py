@@ -301,6 +301,9 @@ def _setup_context(ctx, inputs, output):
     # the gradient of a container goes out at its logical dtype unless the context names one
     ctx.logical = (w13_experts.dtype if w13_experts.dtype != torch.float8_e4m3fn else torch.bfloat16)
     ctx.mark_non_differentiable(counts, logits, route_weights, route_ids, order, offsets, slots, h13)
+    # an output without a cotangent arrives as None, not as a tensor of zeros: those of h13 alone
+    # were a pass over [rows, 2F] bf16 in every backward
+    ctx.set_materialize_grads(False)
     ctx.components = len(weight_components)
 
 
