@@ -430,4 +430,26 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float scale) {
   return make_uint2(w[0], w[1]);
 }
 
+// Position of tile number t in an m_tiles x n_tiles grid that is walked in bands of `band` rows of
+// tiles: inside a band the row runs fastest, so the tiles in flight at one time form a block of
+// about `band` rows by (CTAs / band) columns.  band <= 1 is the plain order, columns fastest.
+// (`tile_band` on the host says which and why.)
+struct TilePos {
+  int m, n;
+};
+__device__ __forceinline__ TilePos banded_tile(int t, int m_tiles, int n_tiles, int band) {
+  TilePos c;
+  if (band <= 1) {
+    c.m = t / n_tiles;
+    c.n = t - c.m * n_tiles;
+  } else {
+    const int first = t / (band * n_tiles) * band;
+    const int rem = t - first * n_tiles;
+    const int height = min(band, m_tiles - first);
+    c.n = rem / height;
+    c.m = first + rem - c.n * height;
+  }
+  return c;
+}
+
 }  // namespace b200

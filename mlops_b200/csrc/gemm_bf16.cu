@@ -43,6 +43,7 @@ struct GemmBf16Params {
   const int* offsets;
   int groups, N, K, rows_total;
   int weights;  // group g multiplies weight matrix g % weights
+  int band;     // M tiles walked together before the next column of tiles (banded_tile)
   float alpha;  // d = alpha * (a @ op(b)) + addend
   int* status;
 };
@@ -139,7 +140,8 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     int group, m0, rows_valid, n0;
   };
   auto locate = [&](int t) {
-    const int mt = t / num_n_tiles;
+    const TilePos pos = banded_tile(t, *total_m_tiles_s, num_n_tiles, p.band);
+    const int mt = pos.m;
     int lo = 0, hi = groups - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -150,7 +152,7 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     c.group = lo;
     c.m0 = offs[lo] + (mt - m_tile_start[lo]) * kBfBlockM;
     c.rows_valid = min(kBfBlockM, offs[lo + 1] - c.m0);
-    c.n0 = (t - mt * num_n_tiles) * kBfBlockN;
+    c.n0 = pos.n * kBfBlockN;
     return c;
   };
 
@@ -359,6 +361,7 @@ extern "C" int b200moe_grouped_gemm_bf16(const void* a, long long lda, const voi
   p.K = K;
   p.rows_total = (int)rows_total;
   p.weights = weights;
+  p.band = tile_band(2LL * N * K);
   p.alpha = alpha;
   p.status = status;
   // upper bound of the tile count: every group may end in a partial tile

@@ -139,6 +139,7 @@ struct GemmFp8Params {
   long long out_rows;  // rows of d (row_map) or of out_f32 (row_token): targets outside are skipped
   int sched_slot;      // slot of g_tile_counter, or -1: tiles by CTA index
   int wide_store;      // d's base and row pitch are multiples of 32 bytes: 32-byte stores per lane
+  int band;            // M tiles walked together before the next column of tiles (banded_tile)
   int tma_store;       // tmap_d describes d: full groups of 32 rows leave through TMA stores
   int* status;
 #ifdef B200_GEMM_TRACE
@@ -248,7 +249,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 22);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   int* total_m_tiles_s = abort_flag + 1;
-  int* sched_tile = total_m_tiles_s + 1;  // [4][4]: tile, its first row, rows that belong to the group, group
+  int* sched_tile = total_m_tiles_s + 1;  // [4][4]: first column, first row, rows that belong to the group, group
   int* m_tile_start = reinterpret_cast<int*>(smem + Cfg::kTileBytes + Cfg::kBarBytes);  // [groups+1]
   int* offs = m_tile_start + (kMaxGroups + 1);                                          // [groups+1]
   // Single-CTA form: warp 2 brings the two scales of every K block from global memory into a ring
@@ -360,9 +361,9 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
   // Tiles are handed out by a global counter, not by stride: a CTA that becomes resident late
   // (its SM was busy with another kernel, e.g. a collective) simply takes fewer tiles, and no
   // tile waits for a CTA that has not started.  The producer draws the numbers and publishes
-  // them, one tile ahead, in a four-slot ring in shared memory; -1 ends the sequence.
-  // `tile_at(i)`: the i-th tile of this CTA (warp-wide call; lane 0 waits); `done_with(i)`
-  // lets the slot be reused.  -2: the wait gave up.
+  // them, one tile ahead, in a four-slot ring in shared memory.
+  // `tile_at(i)`: the first column of this CTA's i-th tile (warp-wide call; lane 0 waits), -1 after
+  // the last one, -2 when the wait gave up; `done_with(i)` lets the slot be reused.
   // The producer locates a tile's rows (a binary search over the groups) once and publishes the
   // answer with the number, so the other roles do not repeat the search at every tile boundary.
   auto tile_at = [&](uint32_t i, TileCoord* where = nullptr) -> int {
@@ -405,12 +406,17 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                    : (int)(blockIdx.x + (drawn++) * gridDim.x);
         return t < total_tiles ? t : -1;
       };
-      auto publish = [&](int t) {
+      auto publish = [&](int t, int& n0, TileCoord& where) {
         const uint32_t slot = published & 3;
         if (!mbar_wait(&sched_empty[slot], ((published >> 2) & 1) ^ 1, abort_flag, p.status, 8)) return false;
-        TileCoord where = {0, 0, 0};
-        if (t >= 0) where = locate(t / num_n_tiles);
-        sched_tile[slot * 4 + 0] = t;
+        where = {0, 0, 0};
+        n0 = -1;
+        if (t >= 0) {
+          const TilePos pos = banded_tile(t, *total_m_tiles_s, num_n_tiles, p.band);
+          where = locate(pos.m);
+          n0 = pos.n * kTileStep;
+        }
+        sched_tile[slot * 4 + 0] = n0;
         sched_tile[slot * 4 + 1] = where.m0;
         sched_tile[slot * 4 + 2] = where.rows_valid;
         sched_tile[slot * 4 + 3] = where.group;
@@ -418,15 +424,13 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
         ++published;
         return true;
       };
-      int t = draw();
-      ok = publish(t);
-      while (ok && t >= 0) {
-        const int t_next = draw();
-        if (!publish(t_next)) { ok = false; break; }  // the epilogue looks one tile ahead
-        const int mt = t / num_n_tiles;
-        const int n0 = (t - mt * num_n_tiles) * kTileStep;
-        const TileCoord c = locate(mt);
-        t = t_next;
+      int n_next;
+      TileCoord c_next;
+      ok = publish(draw(), n_next, c_next);
+      while (ok && n_next >= 0) {
+        const int n0 = n_next;
+        const TileCoord c = c_next;
+        if (!publish(draw(), n_next, c_next)) { ok = false; break; }  // the epilogue looks one tile ahead
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
@@ -520,7 +524,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (t == -2) ok = false;
       else done_with(tile_i);
       if (t < 0) break;
-      const int n0 = (t % num_n_tiles) * kTileStep;
+      const int n0 = t;
       // lane l holds the scales of rows l, l + 32, l + 64, l + 96 of the tile; lanes 0-3 also the
       // weight-block scales: [0], [1] of the columns of epilogue half 0, 1; [2], [3] of their up
       // columns (fused SwiGLU form).  Two K blocks per round of loads: this warp lives on 40
@@ -689,9 +693,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const float* bs_ptr;
       const float* bs_ptr_up;
     };
-    auto describe = [&](int t, const TileCoord& c) {
+    auto describe = [&](int n0, const TileCoord& c) {
       EpiTile e;
-      const int n0 = (t % num_n_tiles) * kTileStep;
       e.rows_valid = c.rows_valid;
       e.grow = c.m0 + row_in_tile;
       e.col0 = EPI == 1 ? n0 + half * 64 : n0 + half * kCols;
@@ -1310,6 +1313,7 @@ static int grouped_gemm_fp8_impl(const void* a, long long lda, const float* a_sc
   p.K = K;
   p.rows_total = (int)rows_total;
   p.weights = weights;
+  p.band = tile_band((long long)N * K);
   p.act_q = nullptr;
   p.ldq = 0;
   p.act_scale = nullptr;
@@ -1487,6 +1491,7 @@ extern "C" int b200moe_grouped_gemm_fp8_swiglu(const void* a, long long lda, con
   p.K = K;
   p.rows_total = (int)rows_total;
   p.weights = weights;
+  p.band = tile_band((long long)N * K);
   p.act_q = reinterpret_cast<uint8_t*>(act_q);
   p.ldq = ldq;
   p.act_scale = act_scale;

@@ -44,6 +44,7 @@ struct WgradParams {
   // X ([groups, N]); the product of a group is multiplied by g_scale[m] * x_scale[n] at the store.
   const float* g_scale;
   const float* x_scale;
+  int band;        // pair kernel: M tiles of a group walked together before the next column of tiles (banded_tile)
   int wide_store;  // the output's base and row pitch are multiples of 32 bytes: 32-byte stores
 };
 
@@ -585,8 +586,9 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
       for (long long t = pair; t < total_tiles && ok; t += num_pairs) {
         const int g = (int)(t / tiles_per_group);
         const int rem = (int)(t - (long long)g * tiles_per_group);
-        const int m0 = (rem / n_tiles) * kPairBlockM + (int)rank * 128;
-        const int n0 = (rem % n_tiles) * kWgBlockN + (int)rank * 128;
+        const TilePos pos = banded_tile(rem, m_tiles, n_tiles, p.band);
+        const int m0 = pos.m * kPairBlockM + (int)rank * 128;
+        const int n0 = pos.n * kWgBlockN + (int)rank * 128;
         for (int seg = 0; seg < p.segments && ok; ++seg) {
           int lo, hi;
           group_range(g, seg, lo, hi);
@@ -712,8 +714,9 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
     for (long long t = pair; t < total_tiles && ok; t += num_pairs) {
       const int g = (int)(t / tiles_per_group);
       const int rem = (int)(t - (long long)g * tiles_per_group);
-      const int m0 = (rem / n_tiles) * kPairBlockM + (int)rank * 128;
-      const int n0 = (rem % n_tiles) * kWgBlockN;
+      const TilePos pos = banded_tile(rem, m_tiles, n_tiles, p.band);
+      const int m0 = pos.m * kPairBlockM + (int)rank * 128;
+      const int n0 = pos.n * kWgBlockN;
       bool has_rows = false;
       for (int seg = 0; seg < p.segments; ++seg) {
         int lo, hi;
@@ -861,6 +864,7 @@ static int grouped_wgrad_impl(const void* g, long long ldg, const void* x, long 
   p.rows_total = (int)rows_total;
   p.segments = segments;
   p.status = status;
+  p.band = tile_band(2 * rows_total / groups * N);
   p.scale = scale;
   p.accumulate = accumulate;
   p.g_scale = nullptr;
@@ -941,6 +945,7 @@ extern "C" int b200moe_grouped_wgrad_fp8(const void* g, long long ldg, const flo
   p.rows_total = (int)rows_total;
   p.segments = segments;
   p.status = status;
+  p.band = tile_band(2 * rows_total / groups * N);
   p.scale = scale;
   p.accumulate = accumulate;
   p.g_scale = g_scale;

@@ -26,6 +26,9 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapFloatOOBfill);
 
 EncodeTiledFn get_encode_tiled();
+// Rows of tiles a GEMM walks together (banded_tile): `bytes` is what one row of tiles reads of the
+// operand that runs along it (a group's whole weight, or its rows of X in a weight gradient).
+int tile_band(long long bytes);
 int sm_count_device();      // SM count of the current device (cached per device)
 int sm_count();             // CTAs a persistent kernel may launch: the SM count, or the limit below
 void set_cta_limit(int n);  // n > 0: persistent kernels launch at most n CTAs; 0: no limit

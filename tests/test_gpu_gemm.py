@@ -612,3 +612,35 @@ def test_tma_store_and_register_store_write_the_same_bytes():
         assert float(line[2]) > 0
         digests.append(line[1])
     assert digests[0] == digests[1]
+
+
+@pytest.mark.parametrize("counts", [[2181, 0, 7], [300, 1900]])
+def test_banded_tile_order_covers_the_same_tiles(counts):
+    """Wide operands (over 40 MB per group) walk their tiles in bands of 16 rows; narrow slices of
+    the same operands do not. Bands that end early (18 and 19 rows of tiles here) included, the
+    products are the same bytes."""
+    ops = _ops()
+    rows, k, n, step = sum(counts), 4096, 10752, 3584
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV, dtype=torch.bfloat16)  # noqa: E731
+    offsets = torch.tensor([0, *torch.tensor(counts).cumsum(0).tolist()], dtype=torch.int32, device=DEV)
+    x, w = randn(rows, k), randn(len(counts), n, k)
+    a_q, a_s = ops.quantize_rows(x)
+    for mn in (False, True):
+        b = w.transpose(1, 2).contiguous() if mn else w
+        part = lambda t, lo, s=1: (t[:, :, lo // s:(lo + step) // s] if mn  # noqa: E731
+                                   else t[:, lo // s:(lo + step) // s]).contiguous()
+        b_q, b_s = ops.quantize_blocks(b)
+        whole = ops.grouped_gemm_fp8(a_q, a_s, b_q, b_s, offsets, b_mn_major=mn)
+        plain = ops.grouped_gemm_bf16(x, b, offsets, b_mn_major=mn)
+        for lo in range(0, n, step):
+            assert torch.equal(whole[:, lo:lo + step], ops.grouped_gemm_fp8(
+                a_q, a_s, part(b_q, lo), part(b_s, lo, 128), offsets, b_mn_major=mn))
+            assert torch.equal(plain[:, lo:lo + step], ops.grouped_gemm_bf16(x, part(b, lo), offsets, b_mn_major=mn))
+    # the weight gradient bands by the average group: one group of the long table, 6144 rows
+    long, m = torch.tensor([0, 6144], dtype=torch.int32, device=DEV), 17 * 256 + 8
+    left, right = randn(6144, m), randn(6144, 3584)
+    whole = ops.grouped_wgrad(left, right, long, 1)
+    for lo in range(0, 3584, 512):
+        assert torch.equal(whole[:, :, lo:lo + 512], ops.grouped_wgrad(left, right[:, lo:lo + 512].contiguous(), long, 1))
+    ops.check_status(DEV)
