@@ -61,6 +61,22 @@ def test_route_ids_bit_exact_on_seeded_logits(tokens, experts, top_k, mode, n_gr
     torch.testing.assert_close(w.cpu(), w_ref, rtol=2e-6, atol=1e-7)
 
 
+@pytest.mark.parametrize("experts,top_k,n_group,topk_group", [(1, 1, 1, 1), (33, 5, 3, 2), (64, 6, 32, 5), (256, 8, 8, 4),
+                                                              (1024, 32, 32, 31), (40, 3, 40, 40), (12, 2, 12, 3)])
+@pytest.mark.parametrize("mode", ["softmax_then_topk", "topk_then_softmax", "sigmoid_noaux_tc"])
+def test_route_breaks_ties_like_a_stable_sort(experts, top_k, n_group, topk_group, mode):
+    """Logits on a coarse grid (every row full of ties, both zeros among them): the ids are those of
+    a stable descending sort, groups of one expert and of many included."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(experts)
+    logits = torch.randint(-3, 4, (257, experts), generator=g) * 0.5
+    logits[::3] *= -1.0  # 0 becomes -0
+    w_ref, id_ref = O.route(logits, top_k, mode, n_group=n_group, topk_group=topk_group)
+    w, ids = ops.route_topk(logits.to(DEV), top_k, mode, n_group=n_group, topk_group=topk_group)
+    assert torch.equal(ids.cpu(), id_ref)
+    torch.testing.assert_close(w.cpu(), w_ref, rtol=2e-6, atol=1e-7)
+
+
 def test_sort_at_full_size_is_a_stable_permutation():
     """Config 5 size (T*K = 524288, E = 128, Zipf-skewed ids): bit-exact against the oracle and
     the size-independent properties (permutation, sortedness, stability, inverse)."""
