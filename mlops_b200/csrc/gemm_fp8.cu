@@ -1029,16 +1029,24 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
           // their maxima through shared memory with a bounded mbarrier wait.
           float amax = 0.f;
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            float gi = __bfloat162float(__float2bfloat16_rn(acc[j]));
-            float ui = __bfloat162float(__float2bfloat16_rn(acc[64 + j]));
-            if (p.limited) {
-              gi = fminf(gi, p.limit);
-              ui = fminf(fmaxf(ui, -p.limit), p.limit);
+          for (int j = 0; j < 64; j += 8) {
+            float g8[8], u8[8], sig[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              g8[i] = __bfloat162float(__float2bfloat16_rn(acc[j + i]));
+              u8[i] = __bfloat162float(__float2bfloat16_rn(acc[64 + j + i]));
+              if (p.limited) {
+                g8[i] = fminf(g8[i], p.limit);
+                u8[i] = fminf(fmaxf(u8[i], -p.limit), p.limit);
+              }
             }
-            const float sig = __frcp_rn(1.0f + expf(-gi));
-            acc[j] = gi * sig * ui;
-            amax = fmaxf(amax, fabsf(acc[j]));
+            if (p.limited) sigmoid8<false>(g8, sig);
+            else sigmoid8<true>(g8, sig);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              acc[j + i] = g8[i] * sig[i] * u8[i];
+              amax = fmaxf(amax, fabsf(acc[j + i]));
+            }
           }
           amax_s[half * 128 + row_in_tile] = amax;
           mbar_arrive(&amax_bar[q]);

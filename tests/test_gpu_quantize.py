@@ -214,3 +214,61 @@ def test_scatter_quantiser_equals_the_gathered_quantiser_bit_for_bit():
     ops.quantize_rows_scatter(x, bad)
     with pytest.raises(NativeError):
         ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("rows", [3, 5000])  # a warp per 256 columns / per row
+@pytest.mark.parametrize("width", [8, 264, 768])
+@pytest.mark.parametrize("limit", [None, 1.3])
+def test_swiglu_over_the_whole_range_of_gates(rows, width, limit):
+    """Gates from 2^-20 to 2^100, infinities and NaN: fp32 SwiGLU rounded once to bf16 is the float64
+    value to one bf16 rounding (2^-8 relative, and 2^-20 of slack for the fp32 steps), values of the
+    two forms (library functions from |g| = 12 on) alike; a NaN stays one."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(rows + width)
+    gate = torch.randn(rows, width, generator=g) * torch.rand(rows, width, generator=g).mul(12).sub(6).exp2()
+    gate[0, :8] = torch.tensor([float("inf"), float("-inf"), float("nan"), 12.0, -12.0, 2.0 ** 100, -88.0, 0.0])
+    up = torch.randn(rows, width, generator=g)
+    h = torch.cat([gate, up], dim=1).bfloat16()
+    _q, _s, act = ops.swiglu_quantize(h.to(DEV), limit=limit, quantized=False, rounded=True)
+    gd, ud = h[:, :width].double(), h[:, width:].double()
+    if limit is not None:
+        cap = torch.tensor(limit, dtype=torch.float32).double()
+        gd, ud = torch.where(gd > cap, cap, gd), ud.clamp(-cap, cap)
+    expected = gd * torch.sigmoid(gd) * ud
+    actual = act.cpu().double()
+    odd = ~expected.isfinite() | gd.isnan() | gd.isinf() | (gd < -80)  # fp32 underflows or overflows there
+    error = (actual - expected).abs()[~odd]
+    assert (error <= expected.abs()[~odd] * (2.0 ** -8 + 2.0 ** -20) + 1e-37).all()
+    if limit is None:
+        assert actual[0, 2].isnan() and actual[0, 0].isinf() and actual[0, 1].isnan()
+
+
+@pytest.mark.parametrize("tokens,width,top_k", [(1, 8, 1), (3, 1032, 2), (70, 2048, 3), (5, 7168, 8), (9, 264, 11)])
+def test_row_kernels_at_the_edges_of_their_pieces(tokens, width, top_k):
+    """Pieces of 512 (scatter quantiser) and 1024 columns (combine, gather), batches of 2, 4 and 8
+    slots: widths that end inside a piece, more slots than a batch, and negative slots, which add
+    nothing. Bit-equal to the oracle (one fp32 sum in slot order, one rounding)."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(tokens * width + top_k)
+    x = torch.randn(tokens, width, generator=g).bfloat16()
+    order = torch.randperm(tokens * top_k, generator=g).to(torch.int32)
+    slots = torch.empty(tokens * top_k, dtype=torch.int32)
+    slots[order.long()] = torch.arange(tokens * top_k, dtype=torch.int32)
+    slots = slots.view(tokens, top_k)
+    rows = x[torch.div(order, top_k, rounding_mode="floor").long()]
+    q_ref, s_ref = O.quantize_rows(rows, mode="1x128")
+    q, s, copy = ops.quantize_rows_scatter(x.to(DEV), slots.to(DEV), with_copy=True)
+    assert torch.equal(q.cpu().view(U8), q_ref.view(U8)) and torch.equal(s.cpu(), s_ref)
+    assert torch.equal(copy.cpu(), rows) and torch.equal(ops.dispatch(x.to(DEV), order.to(DEV), top_k).cpu(), rows)
+    weights = torch.randint(-3, 2, (tokens, top_k), generator=g).float().exp2()  # products are exact, fused or not
+    residual = torch.randn(tokens, width, generator=g).bfloat16()
+    got = ops.combine(rows.to(DEV), slots.to(DEV), weights.to(DEV), residual.to(DEV))
+    assert torch.equal(got.cpu(), O.combine(rows, slots, weights, residual))
+    if top_k > 1:
+        holes = slots.clone()
+        holes[:, 1] = -1
+        zeroed = weights.clone()
+        zeroed[:, 1] = 0
+        got = ops.combine(rows.to(DEV), holes.to(DEV), weights.to(DEV), residual.to(DEV))
+        assert torch.equal(got.cpu(), O.combine(rows, slots, zeroed, residual))
+    ops.check_status(DEV)
