@@ -446,6 +446,89 @@ int b200moe_gather_rows(const void* src, long long lds, long long src_rows, cons
 int b200moe_gather_scalar(const float* values, long long n_values, const int32_t* slots, long long n,
                           float* out, int32_t* status, void* stream);
 
+/*
+ * The block-FP8 layer in one call per direction: the kernels of the entry points above, in the
+ * order a caller would enqueue them.  width and inner are multiples of 128, experts <= 1024,
+ * 0 < top_k <= min(experts, 32), tokens > 0; R = tokens * top_k rows.  Every matrix is dense, every
+ * pointer as aligned as the single entry points want it.
+ *
+ * Forward, after the router GEMM (logits fp32 [tokens, experts]): route, sort, quantise, up GEMM,
+ * SwiGLU, down GEMM, combine, statistics of one sequence (aux, probability_sum).
+ */
+typedef struct b200moe_forward_args {
+  long long tokens;
+  int width, inner, experts, top_k;
+  int mode, n_group, topk_group, limited;
+  float routed_scaling, limit;
+  const void* x;        /* bf16 [tokens, width] */
+  const void* residual; /* bf16 [tokens, width] */
+  const float* logits;
+  const float* bias; /* fp32 [experts] or NULL */
+  const void* w13;   /* E4M3 [experts, 2 inner, width], fp32 scales per 128 x 128 block */
+  const float* w13_scale;
+  const void* w2; /* E4M3 [experts, width, inner] */
+  const float* w2_scale;
+  float* route_weights; /* results: [tokens, top_k] */
+  int32_t* ids;         /* [tokens, top_k] */
+  int32_t* order;       /* [R] */
+  int32_t* offsets;     /* [experts + 1] */
+  int32_t* slots;       /* [tokens, top_k] */
+  long long* counts;    /* [experts] */
+  void* h13;            /* bf16 [R, 2 inner] */
+  void* output;         /* bf16 [tokens, width] */
+  float* aux;
+  float* probability_sum; /* [experts] */
+  void* x_q;              /* scratch: E4M3 [R, width] */
+  void* act_q;            /* E4M3 [R, inner] */
+  void* expert_rows;      /* bf16 [R, width] */
+  void* workspace;        /* b200moe_forward_workspace_bytes, 256-byte aligned */
+  int32_t* status;
+} b200moe_forward_args;
+long long b200moe_forward_workspace_bytes(long long tokens, int width, int inner, int experts, int top_k);
+int b200moe_forward_fp8(const b200moe_forward_args* args, void* stream);
+
+/*
+ * Backward up to the gradient of the logits: input gradient of the experts (grad_x, without the
+ * router's share), weight gradients (NULL: not wanted), gradient of the logits in fp32 and as two
+ * bf16 pieces.  grad_aux (device scalar) and grad_probability_sum may be NULL.
+ */
+typedef struct b200moe_backward_args {
+  long long tokens;
+  int width, inner, experts, top_k;
+  int mode, limited, weight_gradients_fp32;
+  float limit;
+  const void* grad_output; /* bf16 [tokens, width] */
+  const float* grad_aux;
+  const float* grad_probability_sum;
+  const void* x;
+  const void* w13;
+  const float* w13_scale;
+  const void* w2;
+  const float* w2_scale;
+  const float* logits; /* results of the forward pass */
+  const float* route_weights;
+  const int32_t* ids;
+  const int32_t* order;
+  const int32_t* offsets;
+  const int32_t* slots;
+  const void* h13;
+  void* grad_x;            /* bf16 [tokens, width] */
+  float* grad_logits;      /* [tokens, experts] */
+  void* grad_logits_high;  /* bf16 [tokens, experts] */
+  void* grad_logits_low;
+  void* grad_w13; /* [experts, 2 inner, width], bf16 or fp32; NULL: not wanted */
+  void* grad_w2;  /* [experts, width, inner] */
+  void* dy_q;     /* scratch: E4M3 [R, width] */
+  void* rows;     /* bf16 [R, width] */
+  void* r;        /* bf16 [R, inner] */
+  void* gh_q;     /* E4M3 [R, 2 inner] */
+  void* gh;       /* bf16 [R, 2 inner]; may be NULL when grad_w13 is */
+  void* workspace; /* b200moe_backward_workspace_bytes, 256-byte aligned */
+  int32_t* status;
+} b200moe_backward_args;
+long long b200moe_backward_workspace_bytes(long long tokens, int width, int inner, int experts, int top_k);
+int b200moe_backward_fp8(const b200moe_backward_args* args, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

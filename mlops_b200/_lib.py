@@ -29,6 +29,30 @@ LL = c_longlong
 I = c_int
 F = c_float
 
+
+
+class ForwardArgs(ctypes.Structure):
+    """`b200moe_forward_args`"""
+
+    _fields_ = [("tokens", LL)] + [(n, I) for n in (
+        "width", "inner", "experts", "top_k", "mode", "n_group", "topk_group", "limited")] + [
+        ("routed_scaling", F), ("limit", F)] + [(n, P) for n in (
+            "x", "residual", "logits", "bias", "w13", "w13_scale", "w2", "w2_scale", "route_weights", "ids", "order",
+            "offsets", "slots", "counts", "h13", "output", "aux", "probability_sum", "x_q", "act_q", "expert_rows",
+            "workspace", "status")]
+
+
+class BackwardArgs(ctypes.Structure):
+    """`b200moe_backward_args`"""
+
+    _fields_ = [("tokens", LL)] + [(n, I) for n in (
+        "width", "inner", "experts", "top_k", "mode", "limited", "weight_gradients_fp32")] + [("limit", F)] + [
+        (n, P) for n in (
+            "grad_output", "grad_aux", "grad_probability_sum", "x", "w13", "w13_scale", "w2", "w2_scale", "logits",
+            "route_weights", "ids", "order", "offsets", "slots", "h13", "grad_x", "grad_logits", "grad_logits_high",
+            "grad_logits_low", "grad_w13", "grad_w2", "dy_q", "rows", "r", "gh_q", "gh", "workspace", "status")]
+
+
 # name -> (restype, argtypes); one entry per declaration in include/b200moe.h
 SIGNATURES = {
     "b200moe_route_topk": (I, [P, LL, I, I, I, I, P, I, I, F, P, P, P]),
@@ -76,6 +100,10 @@ SIGNATURES = {
     "b200moe_gather_rows": (I, [P, LL, LL, P, I, LL, I, P, LL, P, P]),
     "b200moe_peer_dispatch_rows": (I, [P, LL, LL, P, LL, I, P, LL, LL, P, P, I, P, P]),
     "b200moe_build_copies": (I, [P, P, I, I, I, I, P, P, P, P, P, P]),
+    "b200moe_forward_workspace_bytes": (LL, [LL, I, I, I, I]),
+    "b200moe_forward_fp8": (I, [P, P]),
+    "b200moe_backward_workspace_bytes": (LL, [LL, I, I, I, I]),
+    "b200moe_backward_fp8": (I, [P, P]),
     "b200moe_gather_scalar": (I, [P, LL, P, LL, P, P, P]),
 }
 

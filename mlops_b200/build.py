@@ -60,7 +60,7 @@ def build(force: bool = False, verbose: bool = False, defines=(), output: Path |
     """Compile and link the library when a source changed; return its path. `defines`
     (`NAME=VALUE` strings) and `output` build a variant beside the shipped library."""
     srcs = sources()
-    headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h"))
+    headers = [*sorted(CSRC.glob("*.cuh")), *sorted(CSRC.glob("*.h")), PACKAGE_DIR.parent / "include" / "b200moe.h"]
     variant = bool(defines) or output is not None
     library = Path(output) if output is not None else LIBRARY
     build_dir = BUILD_DIR / ("variant_" + hashlib.sha256(" ".join(defines).encode()).hexdigest()[:8]) if variant \

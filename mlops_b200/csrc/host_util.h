@@ -29,6 +29,13 @@ EncodeTiledFn get_encode_tiled();
 // Rows of tiles a GEMM walks together (banded_tile): `bytes` is what one row of tiles reads of the
 // operand that runs along it (a group's whole weight, or its rows of X in a weight gradient).
 int tile_band(long long bytes);
+// b200moe_routing_gradient, with the gradient written as two bf16 pieces [tokens, experts] as well
+// (high + low; both or neither).
+int launch_routing_gradient(const float* logits, long long ld, long long tokens, int experts, int top_k, int mode,
+                            const int32_t* ids, const float* route_weights, const float* grad_route_weights,
+                            const float* grad_aux, const float* frequency, float aux_scale,
+                            const float* grad_probability_sum, float* grad_logits, long long ldg, void* high,
+                            void* low, cudaStream_t s);
 int sm_count_device();      // SM count of the current device (cached per device)
 int sm_count();             // CTAs a persistent kernel may launch: the SM count, or the limit below
 void set_cta_limit(int n);  // n > 0: persistent kernels launch at most n CTAs; 0: no limit

@@ -231,19 +231,19 @@ swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h13, long long ldh, long l
 // (reference: src/mlops/kernels/quack_moe/swiglu_rows.py:100-199)
 // gh_bf16 may alias h13 (the gradient written over the saved pre-activation): each thread reads
 // the sixteen h13 values of an iteration before it stores the sixteen gradients to the same
-// addresses, and no other thread touches them.
+// addresses, and no other thread touches them; act_scaled may alias r in the same way.
 // One warp per row (the dot product stays in the warp); the next 256 columns are loaded while
 // these are worked on.  32768 rows of F = 14336 with every output: 1.09 ms (6.0 TB/s); 1.36 ms with
 // 77 scalar instructions a value, which kept the kernel issue-bound.
 template <bool LIMITED>
 __global__ void __launch_bounds__(kRowWarps * 32)
 dswiglu_routed_kernel(const __nv_bfloat16* h13, long long ldh,  // may be the same buffer as gh_bf16
-                      const __nv_bfloat16* __restrict__ rmat, long long ldr,
+                      const __nv_bfloat16* rmat, long long ldr,       // may be the same buffer as act_scaled
                       const float* __restrict__ route_weights, long long n_weights,
                       const int* __restrict__ order, long long rows, int F, float* __restrict__ dscore,
                       uint8_t* __restrict__ gh_q, long long ldq, float* __restrict__ gh_scales,
                       long long s_row, long long s_kb, __nv_bfloat16* gh_bf16,
-                      long long ldg, __nv_bfloat16* __restrict__ act_scaled, long long lda, float limit,
+                      long long ldg, __nv_bfloat16* act_scaled, long long lda, float limit,
                       int* status) {
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);

@@ -107,7 +107,8 @@ routing_gradient_kernel(const float* __restrict__ logits, long long ld, long lon
                         const int* __restrict__ ids, const float* __restrict__ weights,
                         const float* __restrict__ grad_weights, const float* __restrict__ grad_aux,
                         const float* __restrict__ frequency, float aux_scale,
-                        const float* __restrict__ grad_psum, float* __restrict__ out, long long ldo) {
+                        const float* __restrict__ grad_psum, float* __restrict__ out, long long ldo,
+                        __nv_bfloat16* __restrict__ high, __nv_bfloat16* __restrict__ low) {
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * kStatWarps + (threadIdx.x >> 5);
   if (t >= tokens) return;
@@ -195,8 +196,16 @@ routing_gradient_kernel(const float* __restrict__ logits, long long ld, long lon
   }
   float* orow = out + t * ldo;
 #pragma unroll
-  for (int j = 0; j < EPL; ++j)
-    if (j * 32 + lane < E) orow[j * 32 + lane] = d[j];
+  for (int j = 0; j < EPL; ++j) {
+    const int e = j * 32 + lane;
+    if (e >= E) continue;
+    orow[e] = d[j];
+    if (high != nullptr) {  // the gradient as two bf16 pieces, operands of the router's own GEMMs
+      const __nv_bfloat16 top = __float2bfloat16_rn(d[j]);
+      high[t * E + e] = top;
+      low[t * E + e] = __float2bfloat16_rn(d[j] - __bfloat162float(top));
+    }
+  }
 }
 
 static long long stat_blocks(long long tokens) {
@@ -248,19 +257,30 @@ extern "C" int b200moe_routing_gradient(const float* logits, long long ld, long 
                                         const float* grad_route_weights, const float* grad_aux,
                                         const float* frequency, float aux_scale, const float* grad_probability_sum,
                                         float* grad_logits, long long ldg, void* stream) {
+  return launch_routing_gradient(logits, ld, tokens, experts, top_k, mode, ids, route_weights, grad_route_weights,
+                                 grad_aux, frequency, aux_scale, grad_probability_sum, grad_logits, ldg, nullptr,
+                                 nullptr, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int b200::launch_routing_gradient(const float* logits, long long ld, long long tokens, int experts, int top_k, int mode,
+                                  const int32_t* ids, const float* route_weights, const float* grad_route_weights,
+                                  const float* grad_aux, const float* frequency, float aux_scale,
+                                  const float* grad_probability_sum, float* grad_logits, long long ldg, void* high,
+                                  void* low, cudaStream_t s) {
   if (!logits || !ids || !grad_route_weights || !grad_logits || tokens < 0 || experts <= 0 || top_k <= 0 ||
       mode < 0 || mode > 2)
     return B200MOE_ERR_ARG;
-  if (mode != 1 && !route_weights) return B200MOE_ERR_ARG;
+  if ((mode != 1 && !route_weights) || (high == nullptr) != (low == nullptr)) return B200MOE_ERR_ARG;
   if (experts > 1024 || top_k > 32) return B200MOE_ERR_LIMIT;
   if (tokens == 0) return B200MOE_OK;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const unsigned grid = (unsigned)((tokens + kStatWarps - 1) / kStatWarps);
 #define CALL_GRADIENT(EPL)                                                                                 \
   routing_gradient_kernel<EPL><<<grid, kStatWarps * 32, 0, s>>>(logits, ld, tokens, experts, top_k, mode,  \
                                                                ids, route_weights, grad_route_weights,    \
                                                                grad_aux, frequency, aux_scale,            \
-                                                               grad_probability_sum, grad_logits, ldg)
+                                                               grad_probability_sum, grad_logits, ldg,    \
+                                                               reinterpret_cast<__nv_bfloat16*>(high),    \
+                                                               reinterpret_cast<__nv_bfloat16*>(low))
   B200_DISPATCH_EPL(experts, CALL_GRADIENT);
 #undef CALL_GRADIENT
   return launch_status();

@@ -37,9 +37,13 @@ def _router_weight_gradient(grad_logits, hidden, dtype):
     """`grad_logits.T @ hidden` with the cotangent carried as two bf16 pieces so an fp32
     master keeps an fp32-quality gradient (reference: src/mlops/kernels/router.py:92-110)."""
     high = grad_logits.to(hidden.dtype)
-    gradient = torch.mm(high.t(), hidden, out_dtype=torch.float32)
     residue = (grad_logits.float() - high.float()).to(hidden.dtype)
-    gradient.add_(torch.mm(residue.t(), hidden, out_dtype=torch.float32))
+    return _router_weight_gradient_of_pieces(high, residue, hidden, dtype)
+
+
+def _router_weight_gradient_of_pieces(high, low, hidden, dtype):
+    gradient = torch.mm(high.t(), hidden, out_dtype=torch.float32)
+    gradient.add_(torch.mm(low.t(), hidden, out_dtype=torch.float32))
     return gradient.to(dtype)
 
 
@@ -163,6 +167,17 @@ def forward_routed(
         residual_flat = residual.reshape_as(h2_flat).contiguous()
         normalized = _normalized_lengths(lengths, h2_flat.shape[0])
         logits = router_logits(h2_flat, router_weight)
+        if (route is None and not bf16_weights and not fuse_swiglu and not fuse_combine
+                and block_n == BLOCK_N_DEFAULT and _one_sequence(routing_mode, normalized)
+                and residual_flat.dtype == torch.bfloat16
+                and ops.whole_layer(h2_flat, w13, w2, experts, int(top_k)) and logits.shape[1] == experts):
+            # one host call for everything that follows
+            bias = None if router_bias is None or router_bias.numel() == 0 else router_bias
+            output, aux, counts, probability_sum, *residuals = ops.forward_fp8(
+                h2_flat, residual_flat, logits, w13, w2, top_k=int(top_k), mode=str(routing_mode), bias=bias,
+                n_group=int(n_group), topk_group=int(topk_group), routed_scaling=float(routed_scaling),
+                limit=None if swiglu_limit is None else float(swiglu_limit))
+            return (output.reshape(original_shape), aux, counts, probability_sum, logits, *residuals)
         if route is None:
             bias = None if router_bias is None or router_bias.numel() == 0 else router_bias
             route_weights, route_ids = ops.route_topk(
@@ -210,6 +225,11 @@ def forward_routed(
             logits, route_ids, counts, routing_mode=str(routing_mode), lengths=normalized, experts=experts
         )
     return (output, aux, counts, probability_sum, logits, route_weights, route_ids, order, offsets, slots, h13)
+
+
+def _one_sequence(routing_mode, lengths):
+    """Whether the routing statistics are those of one sequence (the softmax modes ignore lengths)."""
+    return len(lengths) == 1 or routing_mode != "sigmoid_noaux_tc"
 
 
 def _check_bf16_weights(w13, w2):
@@ -286,6 +306,22 @@ def backward_routed(
         h2_flat = h2.reshape(-1, h2.shape[-1]).contiguous()
         grad_flat = grad_output.reshape_as(h2_flat).contiguous()
         normalized = _normalized_lengths(lengths, h2_flat.shape[0])
+        if (not bf16_weights and weight_grad_operands == "bf16" and block_n == BLOCK_N_DEFAULT
+                and wdtype in (torch.bfloat16, torch.float32)
+                and (grad_aux is None or _one_sequence(routing_mode, normalized))
+                and _saved_as_formed(h2_flat, grad_flat, logits, route_weights, route_ids, order, offsets, slots, h13,
+                                     experts, w2_data.shape[-1], int(top_k))
+                and ops.whole_layer(h2_flat, w13, w2, experts, int(top_k))):
+            grad_h2, _grad_logits, high, low, grad_w13, grad_w2 = ops.backward_fp8(
+                grad_flat, grad_aux, grad_probability_sum, h2_flat, w13, w2, logits, route_weights, route_ids, order,
+                offsets, slots, h13, mode=str(routing_mode), limit=None if swiglu_limit is None else float(swiglu_limit),
+                need_w13=need_w13, need_w2=need_w2, weight_grad_dtype=wdtype)
+            nothing = lambda dtype: torch.empty(0, dtype=dtype, device=h2.device)  # noqa: E731
+            grad_router = nothing(router_weight.dtype) if not need_router else _router_weight_gradient_of_pieces(
+                high, low, h2_flat, router_weight.dtype if router_grad_dtype is None else router_grad_dtype)
+            grad_h2.addmm_(high, getattr(router_weight, "_data", router_weight).to(h2_flat.dtype))
+            return (grad_h2.reshape(original_shape), grad_output.clone(), grad_router,
+                    grad_w13 if need_w13 else nothing(wdtype), grad_w2 if need_w2 else nothing(wdtype))
         counts = (offsets[1:] - offsets[:-1]).long()
 
         if bf16_weights:
@@ -345,6 +381,18 @@ def backward_routed(
         return _finish_backward(grad_h2, grad_output, grad_aux, grad_probability_sum, grad_route_weights,
                                 route_weights, route_ids, logits, counts, routing_mode, normalized, router_weight,
                                 h2_flat, need_router, router_grad_dtype, original_shape, grad_w13, grad_w2)
+
+
+def _saved_as_formed(x, dy, logits, route_weights, route_ids, order, offsets, slots, h13, experts, inner, top_k):
+    """Whether the forward pass's results are the dense tensors it formed (a caller may hand over
+    others, which the step-by-step form converts)."""
+    tokens, width = x.shape
+    rows = tokens * top_k
+    return (dy.dtype == torch.bfloat16 and ops.dense(logits, torch.float32, tokens, experts)
+            and ops.dense(route_weights, torch.float32, tokens, top_k)
+            and ops.dense(route_ids, torch.int32, tokens, top_k) and ops.dense(order, torch.int32, rows)
+            and ops.dense(offsets, torch.int32, experts + 1) and ops.dense(slots, torch.int32, tokens, top_k)
+            and ops.dense(h13, torch.bfloat16, rows, 2 * inner))
 
 
 def _finish_backward(grad_h2, grad_output, grad_aux, grad_probability_sum, grad_route_weights, route_weights,

@@ -172,7 +172,7 @@ def _lora_backward(grad_output, grad_aux, grad_probability_sum, hidden, router_w
         grad_w2 = ops.grouped_wgrad(dy_rows, act_scaled, offsets, experts, wdtype) if need_w2 else empty(wdtype)
 
         grad_logits = layer.routing_gradient(
-            grad_aux, grad_probability_sum, grad_route_weights, weights, ids, logits, counts,
+            provider._given(grad_aux), provider._given(grad_probability_sum), grad_route_weights, weights, ids, logits, counts,
             routing_mode=routing_mode, lengths=tuple(lengths))
         rdtype = router_weight.dtype if weight_grad_dtype is None else weight_grad_dtype
         grad_router = (layer._router_weight_gradient(grad_logits, flat, rdtype) if need_router
@@ -313,10 +313,11 @@ def _autograd_backward(ctx, grad_output, grad_aux, _g_counts, grad_probability_s
     hidden, router_weight = tensors[0], tensors[1]
     if grad_output is None:
         grad_output = torch.zeros_like(hidden)
+    # a cotangent that is not there travels as a tensor without elements
     if grad_aux is None:
-        grad_aux = torch.zeros((), dtype=torch.float32, device=hidden.device)
+        grad_aux = torch.empty(0, dtype=torch.float32, device=hidden.device)
     if grad_probability_sum is None:
-        grad_probability_sum = torch.zeros(router_weight.shape[0], dtype=torch.float32, device=hidden.device)
+        grad_probability_sum = torch.empty(0, dtype=torch.float32, device=hidden.device)
     need = ctx.needs_input_grad
     wdtype = ctx.weight_grad_dtype
     if wdtype is None and ctx.logical != torch.bfloat16:

@@ -10,12 +10,13 @@ Names follow the reference's raw kernel functions (`route`, `sort_assignments`,
 
 from __future__ import annotations
 
+import ctypes
 import functools
 import os
 
 import torch
 
-from ._lib import NativeError, check, lib
+from ._lib import BackwardArgs, ForwardArgs, NativeError, check, lib
 
 ROUTING_MODES = {"topk_then_softmax": 0, "softmax_then_topk": 1, "sigmoid_noaux_tc": 2}
 FP8 = torch.float8_e4m3fn
@@ -898,3 +899,98 @@ def gather_scalar(values, slots):
     )
     _count()
     return out
+
+
+# ------------------------------------------------------- the block-FP8 layer in one call each way
+def dense(t, dtype, *shape):
+    return t.dtype == dtype and t.shape == shape and t.is_contiguous()
+
+
+def whole_layer(x, w13, w2, experts, top_k) -> bool:
+    """Whether the one-call forms below serve these operands; the step-by-step form takes the rest
+    (and any call that is being timed or annotated launch by launch)."""
+    if GEMM_TIMINGS is not None or NVTX:
+        return False
+    (w13_data, w13_scale), (w2_data, w2_scale) = w13, w2
+    width, inner = x.shape[1], w2_data.shape[-1]
+    return (x.dtype == torch.bfloat16 and x.shape[0] > 0 and width % 128 == 0 and inner % 128 == 0 and inner > 0
+            and 0 < top_k <= min(experts, 32) and experts <= 1024 and x.shape[0] * top_k < 2 ** 31
+            and dense(w13_data, FP8, experts, 2 * inner, width) and dense(w2_data, FP8, experts, width, inner)
+            and dense(w13_scale, torch.float32, experts, inner // 64, width // 128)
+            and dense(w2_scale, torch.float32, experts, width // 128, inner // 128))
+
+
+@_on_tensor_device
+def forward_fp8(x, residual, logits, w13, w2, *, top_k, mode, bias=None, n_group=1, topk_group=1, routed_scaling=1.0,
+                limit=None):
+    """The forward pass behind the router GEMM as one host call: `(output, aux, counts,
+    probability_sum, route_weights, route_ids, order, offsets, slots, h13)`, with the statistics of
+    one sequence. The kernels and results of `route_topk`, `sort_assignments`,
+    `quantize_rows_scatter`, `grouped_gemm_fp8`, `swiglu_quantize`, `combine` and
+    `routing_probability_sum` called in that order; for operands `whole_layer` accepts."""
+    (w13_data, w13_scale), (w2_data, w2_scale) = w13, w2
+    device = _need_cuda(x, residual, logits, w13_data, w13_scale, w2_data, w2_scale, bias)
+    tokens, width = x.shape
+    experts, inner = logits.shape[1], w2_data.shape[2]
+    rows = tokens * top_k
+    if not (dense(residual, torch.bfloat16, tokens, width) and dense(logits, torch.float32, tokens, experts)
+            and x.is_contiguous()):
+        raise NativeError("x, residual (bf16) and logits (fp32) must be dense and of one size")
+    if bias is not None:
+        bias = bias.to(torch.float32).contiguous()
+    new = lambda dtype, *shape: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
+    weights, ids = new(torch.float32, tokens, top_k), new(torch.int32, tokens, top_k)
+    order, offsets, slots = new(torch.int32, rows), new(torch.int32, experts + 1), new(torch.int32, tokens, top_k)
+    counts, probability_sum, aux = new(torch.int64, experts), new(torch.float32, experts), new(torch.float32)
+    h13, output = new(torch.bfloat16, rows, 2 * inner), new(torch.bfloat16, tokens, width)
+    x_q, act_q, expert_rows = new(FP8, rows, width), new(FP8, rows, inner), new(torch.bfloat16, rows, width)
+    workspace = new(torch.uint8, lib.b200moe_forward_workspace_bytes(tokens, width, inner, experts, top_k))
+    args = ForwardArgs(
+        tokens, width, inner, experts, top_k, ROUTING_MODES[mode], n_group, topk_group, 0 if limit is None else 1,
+        routed_scaling, 0.0 if limit is None else limit, x.data_ptr(), residual.data_ptr(), logits.data_ptr(),
+        _ptr(bias), w13_data.data_ptr(), w13_scale.data_ptr(), w2_data.data_ptr(), w2_scale.data_ptr(),
+        weights.data_ptr(), ids.data_ptr(), order.data_ptr(), offsets.data_ptr(), slots.data_ptr(), counts.data_ptr(),
+        h13.data_ptr(), output.data_ptr(), aux.data_ptr(), probability_sum.data_ptr(), x_q.data_ptr(),
+        act_q.data_ptr(), expert_rows.data_ptr(), workspace.data_ptr(), status_block(device).data_ptr())
+    check(lib.b200moe_forward_fp8(ctypes.byref(args), _stream()), "forward_fp8")
+    _count(12)
+    return output, aux, counts, probability_sum, weights, ids, order, offsets, slots, h13
+
+
+@_on_tensor_device
+def backward_fp8(grad_output, grad_aux, grad_probability_sum, x, w13, w2, logits, route_weights, route_ids, order,
+                 offsets, slots, h13, *, mode, limit=None, need_w13=True, need_w2=True,
+                 weight_grad_dtype=torch.bfloat16):
+    """The backward pass up to the router as one host call: `(grad_x, grad_logits, high, low,
+    grad_w13, grad_w2)`. `grad_x` lacks the router's share, `high + low` is `grad_logits` as two bf16
+    pieces, a weight gradient nobody needs is None and is not computed. One buffer holds dy, x and
+    the input gradient's rows in turn. For operands `whole_layer` accepts."""
+    (w13_data, w13_scale), (w2_data, w2_scale) = w13, w2
+    device = _need_cuda(grad_output, grad_aux, grad_probability_sum, x, w13_data, w13_scale, w2_data, w2_scale, logits,
+                        route_weights, route_ids, order, offsets, slots, h13)
+    tokens, width = x.shape
+    experts, inner, top_k = logits.shape[1], w2_data.shape[2], route_ids.shape[1]
+    rows = tokens * top_k
+    fp32 = lambda t: None if t is None else t.to(torch.float32).contiguous()  # noqa: E731
+    grad_aux, grad_probability_sum = fp32(grad_aux), fp32(grad_probability_sum)
+    new = lambda dtype, *shape: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
+    grad_x, grad_logits = new(torch.bfloat16, tokens, width), new(torch.float32, tokens, experts)
+    high, low = new(torch.bfloat16, tokens, experts), new(torch.bfloat16, tokens, experts)
+    dy_q, gh_q = new(FP8, rows, width), new(FP8, rows, 2 * inner)
+    row_buffer, r = new(torch.bfloat16, rows, width), new(torch.bfloat16, rows, inner)
+    gh = new(torch.bfloat16, rows, 2 * inner) if need_w13 else None
+    workspace = new(torch.uint8, lib.b200moe_backward_workspace_bytes(tokens, width, inner, experts, top_k))
+    grad_w13 = new(weight_grad_dtype, experts, 2 * inner, width) if need_w13 else None
+    grad_w2 = new(weight_grad_dtype, experts, width, inner) if need_w2 else None
+    args = BackwardArgs(
+        tokens, width, inner, experts, top_k, ROUTING_MODES[mode], 0 if limit is None else 1,
+        1 if weight_grad_dtype == torch.float32 else 0, 0.0 if limit is None else limit, grad_output.data_ptr(),
+        _ptr(grad_aux), _ptr(grad_probability_sum), x.data_ptr(), w13_data.data_ptr(), w13_scale.data_ptr(),
+        w2_data.data_ptr(), w2_scale.data_ptr(), logits.data_ptr(), route_weights.data_ptr(), route_ids.data_ptr(),
+        order.data_ptr(), offsets.data_ptr(), slots.data_ptr(), h13.data_ptr(), grad_x.data_ptr(),
+        grad_logits.data_ptr(), high.data_ptr(), low.data_ptr(), _ptr(grad_w13), _ptr(grad_w2), dy_q.data_ptr(),
+        row_buffer.data_ptr(), r.data_ptr(), gh_q.data_ptr(), _ptr(gh), workspace.data_ptr(),
+        status_block(device).data_ptr())
+    check(lib.b200moe_backward_fp8(ctypes.byref(args), _stream()), "backward_fp8")
+    _count(7 + (1 if need_w2 else 0) + (2 if need_w13 else 0) + (1 if grad_aux is not None else 0))
+    return grad_x, grad_logits, high, low, grad_w13, grad_w2

@@ -23,6 +23,7 @@ the reference asserts that `torch.ops.mlops` holds exactly its own manifest
 from __future__ import annotations
 
 import os
+import sys
 
 import torch
 from torch.utils.flop_counter import register_flop_formula
@@ -58,11 +59,8 @@ def set_weight_gradient_operands(kind: str) -> str:
 # ----------------------------------------------------------------- the reference's contexts
 def _context_weight_gradient_dtype():
     """The reference's `weight_gradients_at(...)` context, when the reference is present."""
-    try:
-        from mlops.dispatch.context import weight_gradient_dtype
-    except ImportError:
-        return None
-    return weight_gradient_dtype()
+    context = sys.modules.get("mlops.dispatch.context")  # one that nobody imported was never entered
+    return None if context is None else context.weight_gradient_dtype()
 
 
 def _context_route_weight_precision() -> str:
@@ -70,11 +68,8 @@ def _context_route_weight_precision() -> str:
     its values give fp32 route weights here, as they do in the reference: "input" means the
     dtype of the logits, and the logits of this path are fp32
     (`src/mlops/kernels/moe_router.py:254-270`, `kernels/router.py:53-64`)."""
-    try:
-        from mlops.kernels.moe_router import current_route_weight_precision
-    except ImportError:
-        return "float32"
-    return current_route_weight_precision()
+    router = sys.modules.get("mlops.kernels.moe_router")
+    return "float32" if router is None else router.current_route_weight_precision()
 
 
 # ------------------------------------------------------------------------------ refusals
@@ -214,6 +209,10 @@ def _moe_fwd_fake(h2, residual, router_weight, w13_experts, w2_experts, router_b
     )
 
 
+def _given(cotangent):
+    return None if cotangent is None or cotangent.numel() == 0 else cotangent
+
+
 def _logical_dtype(weight_grad_dtype, fallback):
     return fallback if weight_grad_dtype is None else weight_grad_dtype
 
@@ -227,12 +226,13 @@ def moe_bwd(grad_output: torch.Tensor, grad_aux: torch.Tensor, grad_probability_
             need_router: bool, need_w13: bool, need_w2: bool,
             weight_components: list[torch.Tensor]) -> _FIVE:
     """`(grad_h2, grad_residual, grad_router, grad_w13, grad_w2)`; a gradient whose `need_*`
-    flag is false is an empty placeholder and its GEMM is not launched."""
+    flag is false is an empty placeholder and its GEMM is not launched. `grad_aux` and
+    `grad_probability_sum` without elements mean none."""
     w13, w2 = _with_scales(w13_experts, w2_experts, weight_components)
     wdtype = _logical_dtype(weight_grad_dtype, torch.bfloat16)
     with torch.cuda.device(h2.device):
         return layer.backward_routed(
-            grad_output, grad_aux, grad_probability_sum, h2, router_weight, w13, w2, logits, route_weights,
+            grad_output, _given(grad_aux), _given(grad_probability_sum), h2, router_weight, w13, w2, logits, route_weights,
             route_ids, order, offsets, slots, h13, top_k=top_k, routing_mode=routing_mode, lengths=lengths,
             weight_grad_dtype=wdtype, router_grad_dtype=weight_grad_dtype, swiglu_limit=swiglu_limit,
             need_router=need_router, need_w13=need_w13, need_w2=need_w2,
@@ -317,10 +317,11 @@ def _autograd_backward(ctx, grad_output, grad_aux, _g_counts, grad_probability_s
     h2, router_weight = tensors[0], tensors[1]
     if grad_output is None:
         grad_output = torch.zeros_like(h2)
+    # a cotangent that is not there travels as a tensor without elements
     if grad_aux is None:
-        grad_aux = torch.zeros((), dtype=torch.float32, device=h2.device)
+        grad_aux = torch.empty(0, dtype=torch.float32, device=h2.device)
     if grad_probability_sum is None:
-        grad_probability_sum = torch.zeros(router_weight.shape[0], dtype=torch.float32, device=h2.device)
+        grad_probability_sum = torch.empty(0, dtype=torch.float32, device=h2.device)
     need = ctx.needs_input_grad
     # None keeps "own dtypes" (the router's; bf16 for E4M3 data); a container whose logical dtype
     # is not bf16 names that dtype, and the router's gradient is brought back to the router's
@@ -501,9 +502,14 @@ def apply(h2, residual, router_weight, w13_experts, w2_experts, *, top_k, routin
     rows = h2.numel() // h2.shape[-1]
     normalized = [rows] if lengths is None else [int(v) for v in lengths]
     bias = router_bias if router_bias is not None else torch.empty(0, dtype=torch.float32, device=h2.device)
+    components = []
+    if type(w13_experts) is BlockFP8Weight and type(w2_experts) is BlockFP8Weight and not torch.is_grad_enabled():
+        # nothing to differentiate: what `_unwrap_containers` would hand on, without its detour
+        components = [w13_experts._scale, w2_experts._scale]
+        w13_experts, w2_experts = w13_experts._data, w2_experts._data
     outputs = moe_fwd(h2, base, router_weight, w13_experts, w2_experts, bias, int(top_k), str(routing_mode),
                       int(n_group), int(topk_group), float(routed_scaling), normalized,
-                      _context_route_weight_precision(), _context_weight_gradient_dtype(), limit, [])
+                      _context_route_weight_precision(), _context_weight_gradient_dtype(), limit, components)
     return outputs[:4]
 
 

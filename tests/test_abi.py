@@ -32,6 +32,26 @@ def test_binding_covers_every_declared_symbol():
     assert sorted(_lib.SIGNATURES) == declared_symbols()
 
 
+def test_argument_structs_are_laid_out_like_the_headers():
+    """Field names, order and types of the argument structs agree with the C declarations."""
+    from mlops_b200 import _lib
+
+    text = re.sub(r"/\*.*?\*/", "", (ROOT / "include" / "b200moe.h").read_text(), flags=re.S)
+    for name, struct in (("b200moe_forward_args", _lib.ForwardArgs), ("b200moe_backward_args", _lib.BackwardArgs)):
+        body = re.search(r"typedef struct %s \{(.*?)\}" % name, text, flags=re.S).group(1)
+        declared = []
+        for line in body.split(";"):
+            if not line.strip():
+                continue
+            if "*" in line:
+                declared.append((line.split("*")[1].strip(), ctypes.c_void_p))
+            else:
+                kind = next(k for k in ("long long", "int", "float") if line.strip().startswith(k))
+                ctype = {"long long": ctypes.c_longlong, "int": ctypes.c_int, "float": ctypes.c_float}[kind]
+                declared += [(n.strip(), ctype) for n in line.strip()[len(kind):].split(",")]
+        assert declared == list(struct._fields_)
+
+
 def test_argument_validation_needs_no_gpu():
     """Entry points reject null pointers and bad sizes before touching the device."""
     from mlops_b200._lib import lib
@@ -42,6 +62,8 @@ def test_argument_validation_needs_no_gpu():
     assert lib.b200moe_grouped_gemm_fp8(None, 0, None, 0, 0, None, None, None, 0, None, 0, None, 1, 1, 0, 8, 16, 0,
                                         128,
                                         None, None) == -1
+    assert lib.b200moe_forward_fp8(None, None) == -1 and lib.b200moe_backward_fp8(None, None) == -1
+    assert lib.b200moe_forward_workspace_bytes(4, 100, 128, 8, 2) == -1
     assert lib.b200moe_combine(None, 0, 0, None, None, None, 0, None, 0, 0, 8, 1, None) == -1
 
 

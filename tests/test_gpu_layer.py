@@ -345,3 +345,46 @@ def test_layer_on_a_device_that_is_not_current():
         outs.append((res[0].cpu(), grads[0].cpu(), grads[3].cpu()))
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("tokens,width,inner,experts,top_k,mode,limit", [
+    (1, 128, 128, 1, 1, "softmax_then_topk", None), (37, 256, 384, 9, 3, "topk_then_softmax", 0.5),
+    (300, 384, 128, 64, 8, "sigmoid_noaux_tc", None), (700, 256, 256, 33, 2, "softmax_then_topk", 2.0)])
+@pytest.mark.parametrize("wdtype", [torch.bfloat16, torch.float32])
+def test_the_one_call_layer_equals_the_step_by_step_form(monkeypatch, tokens, width, inner, experts, top_k, mode,
+                                                         limit, wdtype):
+    """`forward_fp8` / `backward_fp8` against the same layer with every launch timed (which takes the
+    steps one by one): the same bytes, but for the auxiliary loss, an [experts]-sized fp32 sum formed
+    in another order (at most `experts` roundings of 2^-24 apart), and what follows from its
+    cotangent: the experts' frequencies are divided here and multiplied by a reciprocal there, a
+    rounding of 2^-24 that may turn single bf16 roundings of the input gradient (2^-8 of a value, few
+    of them: 2^-10 in the 2-norm) and passes into the router's gradient in two bf16 pieces (2^-14)."""
+    from mlops_b200 import layer, ops
+
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    randn = lambda *s, std=1.0: torch.randn(*s, generator=g, device=DEV) * std  # noqa: E731
+    x, residual, dy = (randn(tokens, width).bfloat16() for _ in range(3))
+    router, bias = randn(experts, width, std=0.1), randn(experts, std=0.01)
+    w13, w2 = ops.quantize_blocks(randn(experts, 2 * inner, width, std=0.1)), ops.quantize_blocks(
+        randn(experts, width, inner, std=0.1))
+    kwargs = dict(top_k=top_k, routing_mode=mode, swiglu_limit=limit)
+    d_aux, d_psum = randn(()), randn(experts)
+
+    def both_passes(**needs):
+        res = layer.forward_routed(x, residual, router, w13, w2, router_bias=bias, **kwargs)
+        grads = [layer.backward_routed(dy, aux, psum, x, router, w13, w2, *res[4:], weight_grad_dtype=wdtype, **kwargs,
+                                       **needs) for aux, psum in ((None, None), (None, d_psum), (d_aux, d_psum))]
+        return res, grads
+
+    for needs in ({}, dict(need_w2=False), dict(need_w13=False, need_router=False)):
+        res, grads = both_passes(**needs)
+        with monkeypatch.context() as patch:
+            patch.setattr(ops, "GEMM_TIMINGS", [])
+            steps, step_grads = both_passes(**needs)
+        torch.testing.assert_close(res[1], steps[1], rtol=experts * 2.0 ** -23, atol=0)
+        for one, other in zip((res[0], *res[2:], *grads[0], *grads[1]), (steps[0], *steps[2:], *step_grads[0], *step_grads[1])):
+            assert one.dtype == other.dtype and torch.equal(one, other)
+        for one, other in zip(grads[2], step_grads[2]):
+            bound = 2.0 ** -14 if one.dtype == torch.float32 else 2.0 ** -10
+            assert (one.float() - other.float()).norm() <= bound * other.float().norm()
+    ops.check_status(DEV)
