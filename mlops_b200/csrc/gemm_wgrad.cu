@@ -489,31 +489,41 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_co
 // leader waits for both reports and issues the MMAs.  The leader's commits arrive on both
 // CTAs' barriers.
 // ---------------------------------------------------------------------------------------
-constexpr int kPairStages = 6;
 constexpr int kPairABytes = 2 * kWgPanelBytes;  // 128 columns of G x 64 K-rows
 constexpr int kPairBBytes = 2 * kWgPanelBytes;  // 128 columns of X x 64 K-rows
-constexpr int kPairTileBytes = kPairStages * (kPairABytes + kPairBBytes);
-constexpr int kPairSmemBytes = 1024 + kPairTileBytes + 512 + 4 * 4104;
+// The output leaves through a buffer per epilogue warp of 32 rows x 32 values; fp32 sums (4 KB a
+// warp) leave room for five operand stages, bf16 ones (2 KB) for six.
+template <typename OutT>
+struct PairCfg {
+  static constexpr int kStages = sizeof(OutT) == 4 ? 5 : 6;
+  static constexpr int kTileBytes = kStages * (kPairABytes + kPairBBytes);
+  static constexpr int kRowBytes = 32 * sizeof(OutT);
+  static constexpr int kStoreBytes = 8 * 32 * kRowBytes;
+  static constexpr int kSmemBytes = 1024 + kTileBytes + kStoreBytes + 512 + 4 * 4104;
+};
 constexpr int kPairBlockM = 256;  // per pair
 
 template <typename OutT>
 __global__ void __launch_bounds__(kWgThreads, 1)
 grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__ CUtensorMap tmap_x,
                           const WgradParams p) {
+  using Cfg = PairCfg<OutT>;
+  constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
-  uint8_t* sB = smem + kPairStages * kPairABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPairTileBytes);
+  uint8_t* sB = smem + kStages * kPairABytes;
+  uint8_t* store_base = smem + Cfg::kTileBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(store_base + Cfg::kStoreBytes);
   uint64_t* landed = bars;                         // [stages] this CTA's TMA bytes
-  uint64_t* ready = bars + kPairStages;            // [stages] leader only: both CTAs' tiles usable
-  uint64_t* empty = bars + 2 * kPairStages;        // [stages] stage consumed (leader's commit, both CTAs)
-  uint64_t* tfull = bars + 3 * kPairStages;        // [2] accumulator complete (leader's commit, both CTAs)
-  uint64_t* tempty = bars + 3 * kPairStages + 2;   // [2] leader only: both CTAs drained the buffer
-  uint64_t* drain = bars + 3 * kPairStages + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kPairStages + 5);
+  uint64_t* ready = bars + kStages;            // [stages] leader only: both CTAs' tiles usable
+  uint64_t* empty = bars + 2 * kStages;        // [stages] stage consumed (leader's commit, both CTAs)
+  uint64_t* tfull = bars + 3 * kStages;        // [2] accumulator complete (leader's commit, both CTAs)
+  uint64_t* tempty = bars + 3 * kStages + 2;   // [2] leader only: both CTAs drained the buffer
+  uint64_t* drain = bars + 3 * kStages + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 5);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
-  int* offs_s = reinterpret_cast<int*>(smem + kPairTileBytes + 512);
+  int* offs_s = reinterpret_cast<int*>(store_base + Cfg::kStoreBytes + 512);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -527,7 +537,7 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
   const long long total_tiles = (long long)tiles_per_group * p.groups;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPairStages; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(&landed[s], 1);
       mbar_init(&ready[s], 2);   // one arrival per CTA of the pair
       mbar_init(&empty[s], 1);
@@ -594,8 +604,8 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
           group_range(g, seg, lo, hi);
           const int num_kb = (hi - lo + kWgBlockK - 1) / kWgBlockK;
           for (int kb = 0; kb < num_kb; ++kb, ++it) {
-            const int s = it % kPairStages;
-            const uint32_t ph = (it / kPairStages) & 1;
+            const int s = it % kStages;
+            const uint32_t ph = (it / kStages) & 1;
             if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 31)) { ok = false; break; }
             mbar_arrive_expect_tx(&landed[s], kPairABytes + kPairBBytes);
             const int krow = lo + kb * kWgBlockK;
@@ -609,11 +619,11 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
       }
       if (!ok) {
         const uint32_t issued = it;
-        for (int s = 0; s < kPairStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
           if (issued <= (uint32_t)s) continue;
-          const uint32_t last = ((issued - 1 - s) / kPairStages) * kPairStages + s;
+          const uint32_t last = ((issued - 1 - s) / kStages) * kStages + s;
           const long long start = clock64();
-          while (!mbar_try(&landed[s], (last / kPairStages) & 1) && clock64() - start < 20000000LL) {}
+          while (!mbar_try(&landed[s], (last / kStages) & 1) && clock64() - start < 20000000LL) {}
         }
       }
     }
@@ -628,8 +638,8 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
         group_range(g, seg, lo, hi);
         const int num_kb = (hi - lo + kWgBlockK - 1) / kWgBlockK;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % kPairStages;
-          const uint32_t ph = (it / kPairStages) & 1;
+          const int s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait_warp(&landed[s], ph, abort_flag, p.status, 32)) { ok = false; break; }
           const int valid = hi - lo - kb * kWgBlockK;
           if (valid < kWgBlockK) {
@@ -682,8 +692,8 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
         ++tb;
         if (!mbar_wait(&tempty[buf], aph ^ 1, abort_flag, p.status, 33)) { ok = false; break; }
         for (int done_kb = 0; done_kb < total_kb; ++done_kb, ++it) {
-          const int s = it % kPairStages;
-          const uint32_t ph = (it / kPairStages) & 1;
+          const int s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait(&ready[s], ph, abort_flag, p.status, 34)) { ok = false; break; }
           tc_fence_after_sync();
           const uint64_t adesc = make_smem_desc(smem_u32(sA + s * kPairABytes), kWgPanelBytes, 1024);
@@ -723,7 +733,8 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
         group_range(g, seg, lo, hi);
         has_rows = has_rows || hi > lo;
       }
-      const int m = m0 + q * 32 + lane;
+      const int row0 = m0 + q * 32;  // first of the warp's 32 rows
+      const int m = row0 + lane;
       const int col0 = n0 + half * kCols;
       OutT* orow = out + ((long long)g * p.M + m) * p.N + col0;
       int buf = 0;
@@ -741,22 +752,60 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
         if (has_rows) {
           tmem_ld_32x32(taddr + cc * 32, r);
           tmem_ld_wait();
+          if (cc == kCols / 32 - 1) {  // the warp's part of the accumulator is in registers: hand it back
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(&tempty[buf], 0);
+          }
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
         const int cols = min(32, p.N - (col0 + cc * 32));  // of this chunk inside the matrix (a multiple of 8)
-        if (m < p.M && cols > 0) {
-          float v[32];
+        if (p.accumulate) {
+          if (m < p.M && cols > 0) {
+            float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-          finish32<OutT>(orow + cc * 32, v, cols, p.scale, p.accumulate, p.wide_store != 0);
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            finish32<OutT>(orow + cc * 32, v, cols, p.scale, 1, p.wide_store != 0);
+          }
+          continue;
         }
-      }
-      if (has_rows) {
-        tc_fence_before_sync();
+        // One row per lane would make every store instruction touch 32 rows with a sector each,
+        // some 80 cycles of the SM's memory pipeline: a tile's stores took 10000 cycles (fp32) or
+        // 6500 (bf16), against 2000 of multiplication where an expert has 256 rows.  Through the
+        // warp's buffer (16-byte pieces, swizzled so that both sides are free of bank conflicts)
+        // an instruction writes whole 128-byte (fp32) or 64-byte (bf16) rows: 128 experts of 256 rows,
+        // 1536 x 2048 outputs, fp32 447 -> 338 us, bf16 273 -> 253; 1024 rows of 4096 x 7168 alike.
+        // (The scale is 1 on this path.)
+        constexpr int kRowPieces = Cfg::kRowBytes / 16;
+        auto piece_at = [](int row, int piece) {
+          return row * Cfg::kRowBytes + ((piece ^ (kRowPieces == 8 ? row & 7 : (row >> 1) & 3)) << 4);
+        };
+        uint8_t* buffer = store_base + (warp - 4) * (32 * Cfg::kRowBytes);
+        __syncwarp();  // the previous chunk has been read
+#pragma unroll
+        for (int j = 0; j < kRowPieces; ++j) {
+          uint4 w;
+          if constexpr (sizeof(OutT) == 4) {
+            w = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          } else {
+            w.x = pack_bf16x2(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1]));
+            w.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
+            w.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
+            w.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
+          }
+          *reinterpret_cast<uint4*>(buffer + piece_at(lane, j)) = w;
+        }
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(&tempty[buf], 0);
+        constexpr int kPieceCols = 16 / sizeof(OutT), kRowsPerStore = 32 / kRowPieces;
+        const int piece = lane % kRowPieces;
+        OutT* to = out + ((long long)g * p.M + row0) * p.N + col0 + cc * 32 + piece * kPieceCols;
+#pragma unroll
+        for (int row = lane / kRowPieces; row < 32; row += kRowsPerStore)
+          if (row0 + row < p.M && piece * kPieceCols < cols)
+            *reinterpret_cast<uint4*>(to + (long long)row * p.N) =
+                *reinterpret_cast<const uint4*>(buffer + piece_at(row, piece));
       }
     }
   }
@@ -772,7 +821,7 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
 template <typename OutT>
 static int launch_pair(const CUtensorMap& tg, const CUtensorMap& tx, const WgradParams& p, cudaStream_t s) {
   auto kern = grouped_wgrad_pair_kernel<OutT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) != cudaSuccess)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<OutT>::kSmemBytes) != cudaSuccess)
     return B200MOE_ERR_LAUNCH;
   const long long tiles = (long long)p.groups * ((p.M + kPairBlockM - 1) / kPairBlockM) *
                           ((p.N + kWgBlockN - 1) / kWgBlockN);
@@ -782,7 +831,7 @@ static int launch_pair(const CUtensorMap& tg, const CUtensorMap& tx, const Wgrad
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs));
   cfg.blockDim = dim3(kWgThreads);
-  cfg.dynamicSmemBytes = kPairSmemBytes;
+  cfg.dynamicSmemBytes = PairCfg<OutT>::kSmemBytes;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
