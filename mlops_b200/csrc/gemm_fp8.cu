@@ -220,6 +220,7 @@ __device__ __forceinline__ TileCoord locate_m_tile(int mt, const int* m_tile_sta
 template <int BLOCK_N, bool B_MN_MAJOR, int EPI, bool SPLIT = false, bool PAIR = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
+                        const __grid_constant__ CUtensorMap tmap_a32,  // the same matrix, 32 rows a box
                         const __grid_constant__ CUtensorMap tmap_b,
                         const __grid_constant__ CUtensorMap tmap_d, const GemmFp8Params p) {
   using Cfg = GemmCfg<BLOCK_N, PAIR>;
@@ -297,6 +298,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_a32);
     tma_prefetch_desc(&tmap_b);
   }
   if (warp == 2) {
@@ -430,6 +432,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
       while (ok && n_next >= 0) {
         const int n0 = n_next;
         const TileCoord c = c_next;
+        // Only the 32-row pieces of A that hold rows of the group are loaded; what the others left in
+        // the stage is multiplied into accumulator rows that nobody reads (and the epilogue warps of
+        // those rows hand the accumulator back unread).  256 experts, 64 tokens with 8 experts each:
+        // 4096 x 7168 1132 -> 1061 us, 7168 x 2048 587 -> 552; 8192 tokens 2838 -> 2744, 1590 -> 1509.
+        const int a_pieces = PAIR ? 4 : min(4, (c.rows_valid + 31) / 32);
         if (!publish(draw(), n_next, c_next)) { ok = false; break; }  // the epilogue looks one tile ahead
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % kStages;
@@ -444,8 +451,15 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
             mbar_arrive(&full[s]);
             continue;
           }
-          mbar_arrive_expect_tx(&full[s], Cfg::kABytes + Cfg::kBBytes);
-          tma_load_2d(sA + s * Cfg::kABytes, &tmap_a, &full[s], kb * kBlockK, c.m0);
+          if (a_pieces == 4) {
+            mbar_arrive_expect_tx(&full[s], Cfg::kABytes + Cfg::kBBytes);
+            tma_load_2d(sA + s * Cfg::kABytes, &tmap_a, &full[s], kb * kBlockK, c.m0);
+          } else {
+            mbar_arrive_expect_tx(&full[s], a_pieces * (Cfg::kABytes / 4) + Cfg::kBBytes);
+            for (int i = 0; i < a_pieces; ++i)
+              tma_load_2d(sA + s * Cfg::kABytes + i * (Cfg::kABytes / 4), &tmap_a32, &full[s], kb * kBlockK,
+                          c.m0 + i * 32);
+          }
           if constexpr (PAIR && SPLIT) {
             // this CTA's 64 columns of each 128-column half (two loads of 8 KB)
 #pragma unroll
@@ -748,6 +762,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const EpiTile c = cur_tile;
       const int grow = c.grow;
       const int col0 = c.col0;
+      const bool idle = c.rows_valid <= q * 32;
 #pragma unroll
       for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
       for (int kb0 = 0; kb0 < num_kb && ok; kb0 += kScaleBatch) {
@@ -783,6 +798,15 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
             s_up = EPI == 1 ? sa * slot[130 + half] : s;
           }
           tc_fence_after_sync();
+          if (idle) {  // none of the warp's 32 rows belongs to the group
+            if constexpr (PAIR) {
+              __syncwarp();
+              if (lane == 0) mbar_arrive_remote(&tempty[part], 0);
+            } else {
+              named_arrive(kAccBarrier + part, kRelThreads);
+            }
+            continue;
+          }
           const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BLOCK_N +
                                  (EPI == 1 ? half * 64 : half * kCols);
           // EPI == 1: chunks 0,1 are this thread's 64 gate columns, chunks 2,3 its 64 up columns.
@@ -1138,7 +1162,7 @@ static int sched_slot_of(cudaStream_t stream) {
 
 // The pair form: clusters of two CTAs, one 256 x 256 tile per pair at a time.
 template <bool B_MN, bool SPLIT>
-static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
+static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& ta32, const CUtensorMap& tb, const CUtensorMap& td,
                             const GemmFp8Params& p, cudaStream_t stream) {
   using Cfg = GemmCfg<256, true>;
   auto kern = grouped_gemm_fp8_kernel<256, B_MN, 0, SPLIT, true>;
@@ -1163,12 +1187,12 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, td, q) != cudaSuccess) return B200MOE_ERR_LAUNCH;
+  if (cudaLaunchKernelEx(&cfg, kern, ta, ta32, tb, td, q) != cudaSuccess) return B200MOE_ERR_LAUNCH;
   return launch_status();
 }
 
 template <int BLOCK_N, bool B_MN, int EPI = 0, bool SPLIT = false>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
+static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& ta32, const CUtensorMap& tb, const CUtensorMap& td,
                        const GemmFp8Params& p, cudaStream_t stream) {
   using Cfg = GemmCfg<BLOCK_N>;
   auto kern = grouped_gemm_fp8_kernel<BLOCK_N, B_MN, EPI, SPLIT>;
@@ -1190,7 +1214,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   if (grid < 1) grid = 1;
   GemmFp8Params q = p;
   q.sched_slot = sched_slot_of(stream);
-  kern<<<(unsigned)grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(ta, tb, td, q);
+  kern<<<(unsigned)grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(ta, ta32, tb, td, q);
   return launch_status();
 }
 
@@ -1288,12 +1312,12 @@ static int grouped_gemm_fp8_impl(const void* a, long long lda, const float* a_sc
   if (b_mn_major && (N % 16)) return B200MOE_ERR_ALIGN;
   if (rows_total == 0) return B200MOE_OK;
 
-  CUtensorMap ta, tb;
-  {
+  CUtensorMap ta, ta32, tb;
+  for (int rows : {128, 32}) {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)rows_total};
     uint64_t strides[1] = {(uint64_t)lda};
-    uint32_t box[2] = {128, 128};
-    int r = encode_tensor_map(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a, dims, strides, box,
+    uint32_t box[2] = {128, (uint32_t)rows};
+    int r = encode_tensor_map(rows == 128 ? &ta : &ta32, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B);
     if (r != B200MOE_OK) return r;
   }
@@ -1374,9 +1398,9 @@ static int grouped_gemm_fp8_impl(const void* a, long long lda, const float* a_sc
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (pair && pair_split)
-    return b_mn_major ? launch_gemm_pair<true, true>(ta, tb, td, p, s) : launch_gemm_pair<false, true>(ta, tb, td, p, s);
+    return b_mn_major ? launch_gemm_pair<true, true>(ta, ta32, tb, td, p, s) : launch_gemm_pair<false, true>(ta, ta32, tb, td, p, s);
   if (pair)
-    return b_mn_major ? launch_gemm_pair<true, false>(ta, tb, td, p, s) : launch_gemm_pair<false, false>(ta, tb, td, p, s);
+    return b_mn_major ? launch_gemm_pair<true, false>(ta, ta32, tb, td, p, s) : launch_gemm_pair<false, false>(ta, ta32, tb, td, p, s);
   // the 256-wide tile issues each K block in two halves (B200MOE_GEMM_SPLIT=0: in one piece)
   static const bool split = [] {
     const char* v = getenv("B200MOE_GEMM_SPLIT");
@@ -1384,15 +1408,15 @@ static int grouped_gemm_fp8_impl(const void* a, long long lda, const float* a_sc
   }();
   if (fused) {
     if (split)
-      return b_mn_major ? launch_gemm<256, true, 2, true>(ta, tb, td, p, s) : launch_gemm<256, false, 2, true>(ta, tb, td, p, s);
-    return b_mn_major ? launch_gemm<256, true, 2>(ta, tb, td, p, s) : launch_gemm<256, false, 2>(ta, tb, td, p, s);
+      return b_mn_major ? launch_gemm<256, true, 2, true>(ta, ta32, tb, td, p, s) : launch_gemm<256, false, 2, true>(ta, ta32, tb, td, p, s);
+    return b_mn_major ? launch_gemm<256, true, 2>(ta, ta32, tb, td, p, s) : launch_gemm<256, false, 2>(ta, ta32, tb, td, p, s);
   }
   if (block_n == 128) {
-    return b_mn_major ? launch_gemm<128, true>(ta, tb, td, p, s) : launch_gemm<128, false>(ta, tb, td, p, s);
+    return b_mn_major ? launch_gemm<128, true>(ta, ta32, tb, td, p, s) : launch_gemm<128, false>(ta, ta32, tb, td, p, s);
   }
   if (split)
-    return b_mn_major ? launch_gemm<256, true, 0, true>(ta, tb, td, p, s) : launch_gemm<256, false, 0, true>(ta, tb, td, p, s);
-  return b_mn_major ? launch_gemm<256, true>(ta, tb, td, p, s) : launch_gemm<256, false>(ta, tb, td, p, s);
+    return b_mn_major ? launch_gemm<256, true, 0, true>(ta, ta32, tb, td, p, s) : launch_gemm<256, false, 0, true>(ta, ta32, tb, td, p, s);
+  return b_mn_major ? launch_gemm<256, true>(ta, ta32, tb, td, p, s) : launch_gemm<256, false>(ta, ta32, tb, td, p, s);
 }
 
 extern "C" int b200moe_grouped_gemm_fp8(const void* a, long long lda, const float* a_scale,
@@ -1459,12 +1483,12 @@ extern "C" int b200moe_grouped_gemm_fp8_swiglu(const void* a, long long lda, con
     return B200MOE_ERR_ALIGN;
   if (rows_total == 0) return B200MOE_OK;
   const int N = 2 * F;
-  CUtensorMap ta, tb;
-  {
+  CUtensorMap ta, ta32, tb;
+  for (int rows : {128, 32}) {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)rows_total};
     uint64_t strides[1] = {(uint64_t)lda};
-    uint32_t box[2] = {128, 128};
-    int r = encode_tensor_map(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a, dims, strides, box,
+    uint32_t box[2] = {128, (uint32_t)rows};
+    int r = encode_tensor_map(rows == 128 ? &ta : &ta32, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B);
     if (r != B200MOE_OK) return r;
   }
@@ -1516,7 +1540,7 @@ extern "C" int b200moe_grouped_gemm_fp8_swiglu(const void* a, long long lda, con
   p.status = status;
   B200_SET_TRACE(p);
   B200_SET_WITHHOLD(p);
-  return launch_gemm<256, false, 1>(ta, tb, td, p, reinterpret_cast<cudaStream_t>(stream));
+  return launch_gemm<256, false, 1>(ta, ta32, tb, td, p, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int b200moe_set_cta_limit(int ctas) {
