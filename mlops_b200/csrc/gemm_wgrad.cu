@@ -478,6 +478,311 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_co
 
 
 // ---------------------------------------------------------------------------------------
+// Narrow outputs (the factors of a low-rank adapter): one side of dW[g] is at most 64 wide.  The wide
+// side is always the 128-row operand of the multiplication and the narrow one its N (16 to 64), so a
+// K block is 24 KB of operands (eight stages) and a short multiplication, whichever side of the output
+// is narrow; TRANSPOSED says that the output's rows are the narrow side, and the accumulator is stored
+// column by column (32 lanes, 32 neighbouring values).  Bound by reading the wide operand.
+//
+// Every tile of a group contracts all rows of the group, and groups differ by a factor of a hundred
+// under skewed routing, so the tiles are not dealt out by index.  The CTAs form teams of one per wide
+// tile; a team takes the contiguous range of groups whose work (K blocks, plus kNarrowTileCost per group)
+// falls into its share, and its CTAs walk the same rows side by side, so that HBM sees whole rows (ranges
+// of tiles per CTA were as well balanced but read 256 bytes a row at a time: 594 us for the first below).
+// Measured with 524288 rows Zipf(1.2) over 128 experts, rank 16, in us, 128 x 256 tiles by index -> this:
+//   2048 x 16  694 -> 503 (4.3 TB/s)   16 x 2048  569 -> 505   1536 x 16  604 -> 421   16 x 768  457 -> 421
+// The last two are one group's chain of 1024 K blocks (65536 of the rows), some 780 cycles each.
+// ---------------------------------------------------------------------------------------
+constexpr int kNarrowMax = 64;
+constexpr int kNarrowStages = 8;
+constexpr int kNarrowABytes = 2 * kWgPanelBytes;  // 128 columns of the wide operand x 64 K-rows
+constexpr int kNarrowBBytes = kWgPanelBytes;      // up to 64 columns of the narrow one
+constexpr int kNarrowTileBytes = kNarrowStages * (kNarrowABytes + kNarrowBBytes);
+constexpr int kNarrowTmemCols = 2 * kNarrowMax;
+constexpr int kNarrowTileCost = 6;
+constexpr int kNarrowSmemBytes = 1024 + kNarrowTileBytes + 256 + 8 * (kWgMaxGroups + 2) + 4 * 4104;
+
+template <typename OutT>
+__device__ __forceinline__ void finish1(OutT* dst, float v, float scale, int accumulate) {
+  v = accumulate ? fmaf(scale, v, (float)*dst) : v * scale;
+  *dst = (OutT)v;
+}
+
+template <typename OutT, bool TRANSPOSED>
+__global__ void __launch_bounds__(kWgThreads, 1)
+grouped_wgrad_narrow_kernel(const __grid_constant__ CUtensorMap tmap_wide, const __grid_constant__ CUtensorMap tmap_narrow,
+                            const WgradParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + kNarrowStages * kNarrowABytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kNarrowTileBytes);
+  uint64_t* full = bars;
+  uint64_t* empty = bars + kNarrowStages;
+  uint64_t* tfull = bars + 2 * kNarrowStages;
+  uint64_t* tempty = bars + 2 * kNarrowStages + 2;
+  uint64_t* drain = bars + 2 * kNarrowStages + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kNarrowStages + 5);
+  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+  long long* work = reinterpret_cast<long long*>(smem + kNarrowTileBytes + 256);  // [groups + 1] work before a group
+  int* offs_s = reinterpret_cast<int*>(work + kWgMaxGroups + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int wide = TRANSPOSED ? p.N : p.M, narrow = TRANSPOSED ? p.M : p.N;
+  const int tiles_per_group = (wide + kWgBlockM - 1) / kWgBlockM;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kNarrowStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(&tfull[0], 1);
+    mbar_init(&tfull[1], 1);
+    mbar_init(&tempty[0], 8);
+    mbar_init(&tempty[1], 8);
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmap_wide);
+    tma_prefetch_desc(&tmap_narrow);
+  }
+  if (warp == 2) {
+    tmem_alloc(tmem_slot, kNarrowTmemCols);
+    tmem_relinquish();
+  }
+  __syncthreads();  // abort_flag initialised before the table check may set it
+  // A malformed table (negative, decreasing, past the end) is reported and every range becomes empty.
+  {
+    const int entries = p.segments * p.groups + 1;
+    for (int i = threadIdx.x; i < entries; i += blockDim.x) {
+      const int v = p.offsets[i];
+      const int nxt = i + 1 < entries ? p.offsets[i + 1] : v;
+      if (v < 0 || nxt < v || nxt > p.rows_total) {
+        report_error(p.status, ERR_BAD_OFFSETS, 20, i);
+        *abort_flag = 2;  // not an abort: marks the table as unusable
+      }
+      offs_s[i] = v;
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const bool table_ok = *abort_flag != 2;
+  __syncthreads();
+  if (threadIdx.x == 0) *abort_flag = 0;
+
+  auto group_range = [&](int g, int seg, int& lo, int& hi) {
+    const int at = seg * p.groups + g;
+    lo = offs_s[at];
+    hi = table_ok ? offs_s[at + 1] : lo;
+  };
+  auto group_blocks = [&](int g) {
+    int blocks = 0;
+    for (int seg = 0; seg < p.segments; ++seg) {
+      int lo, hi;
+      group_range(g, seg, lo, hi);
+      blocks += (hi - lo + kWgBlockK - 1) / kWgBlockK;
+    }
+    return blocks;
+  };
+  if (warp == 3) {
+    long long running = 0;
+    for (int base = 0; base < p.groups; base += 32) {
+      const int g = base + lane;
+      const long long mine = g < p.groups ? group_blocks(g) + kNarrowTileCost : 0;
+      long long upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      if (g < p.groups) work[g] = running + upto - mine;
+      running += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (lane == 0) work[p.groups] = running;
+  }
+  __syncthreads();
+  // Team `team` of `teams` works on the groups whose middle lies in its share of the work; this CTA on
+  // wide tiles first_w, first_w + team_size, ...
+  const int team_size = min(tiles_per_group, (int)gridDim.x);
+  const int teams = (int)gridDim.x / team_size, team = (int)blockIdx.x / team_size;
+  const int first_w = (int)blockIdx.x % team_size;
+  auto first_group = [&](int of_team) {
+    int lo = 0, hi = p.groups;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if ((work[mid] + work[mid + 1]) * teams >= 2 * work[p.groups] * of_team) hi = mid;
+      else lo = mid + 1;
+    }
+    return lo;
+  };
+  const int g_begin = team < teams ? first_group(team) : 0;
+  const int my_groups = team < teams ? (team + 1 == teams ? p.groups : first_group(team + 1)) - g_begin : 0;
+  const int my_tiles = my_groups * ((tiles_per_group - first_w + team_size - 1) / team_size);
+  auto tile_group = [&](int t) { return g_begin + t % my_groups; };
+  auto tile_column = [&](int t) { return (first_w + t / my_groups * team_size) * kWgBlockM; };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = 0; t < my_tiles && ok; ++t) {
+        const int g = tile_group(t), w0 = tile_column(t);
+        for (int seg = 0; seg < p.segments && ok; ++seg) {
+          int lo, hi;
+          group_range(g, seg, lo, hi);
+          const int num_kb = (hi - lo + kWgBlockK - 1) / kWgBlockK;
+          for (int kb = 0; kb < num_kb; ++kb, ++it) {
+            const int s = it % kNarrowStages;
+            const uint32_t ph = (it / kNarrowStages) & 1;
+            if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 51)) { ok = false; break; }
+            mbar_arrive_expect_tx(&full[s], kNarrowABytes + kNarrowBBytes);
+            const int krow = lo + kb * kWgBlockK;
+#pragma unroll
+            for (int pnl = 0; pnl < 2; ++pnl)
+              tma_load_2d(sA + s * kNarrowABytes + pnl * kWgPanelBytes, &tmap_wide, &full[s], w0 + pnl * 64, krow);
+            tma_load_2d(sB + s * kNarrowBBytes, &tmap_narrow, &full[s], 0, krow);
+          }
+        }
+      }
+      if (!ok) {
+        const uint32_t issued = it;
+        for (int s = 0; s < kNarrowStages; ++s) {
+          if (issued <= (uint32_t)s) continue;
+          const uint32_t last = ((issued - 1 - s) / kNarrowStages) * kNarrowStages + s;
+          const uint32_t ph = (last / kNarrowStages) & 1;
+          const long long start = clock64();
+          while (!mbar_try(&full[s], ph) && clock64() - start < 20000000LL) {}
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // All 32 lanes stay in the loop: they zero the K tail together; lane 0 issues.
+    const uint32_t idesc = make_idesc(1, 1, 1, 1, kWgBlockM, (narrow + 15) / 16 * 16);
+    uint32_t it = 0, tb = 0;
+    bool ok = true;
+    for (int t = 0; t < my_tiles && ok; ++t) {
+      const int g = tile_group(t);
+      const int total_kb = group_blocks(g);
+      if (total_kb == 0) continue;
+      const int buf = tb & 1;
+      const uint32_t aph = (tb >> 1) & 1;
+      ++tb;
+      if (!mbar_wait_warp(&tempty[buf], aph ^ 1, abort_flag, p.status, 53)) { ok = false; break; }
+      int done_kb = 0;
+      for (int seg = 0; seg < p.segments && ok; ++seg) {
+        int lo, hi;
+        group_range(g, seg, lo, hi);
+        const int num_kb = (hi - lo + kWgBlockK - 1) / kWgBlockK;
+        for (int kb = 0; kb < num_kb; ++kb, ++it, ++done_kb) {
+          const int s = it % kNarrowStages;
+          const uint32_t ph = (it / kNarrowStages) & 1;
+          if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, 52)) { ok = false; break; }
+          const int valid = hi - lo - kb * kWgBlockK;
+          if (valid < kWgBlockK) {
+            // both operands (see the kernel above): two panels of the wide one, one of the narrow one
+            const int nbytes = (kWgBlockK - valid) * 128;
+            for (int pnl = 0; pnl < 3; ++pnl) {
+              uint8_t* base = (pnl < 2 ? sA + s * kNarrowABytes + pnl * kWgPanelBytes : sB + s * kNarrowBBytes) +
+                              valid * 128;
+              for (int o = lane * 16; o < nbytes; o += 32 * 16)
+                *reinterpret_cast<uint4*>(base + o) = make_uint4(0, 0, 0, 0);
+            }
+            fence_proxy_async_smem();
+          }
+          __syncwarp();
+          tc_fence_after_sync();
+          if (lane == 0) {
+            const uint64_t adesc = make_smem_desc(smem_u32(sA + s * kNarrowABytes), kWgPanelBytes, 1024);
+            const uint64_t bdesc = make_smem_desc(smem_u32(sB + s * kNarrowBBytes), kWgPanelBytes, 1024);
+            const uint32_t d_tmem = tmem_base + buf * kNarrowMax;
+#pragma unroll
+            for (int k = 0; k < kWgBlockK / 16; ++k) {
+              const uint64_t step = (uint64_t)((k * 16 * 128) >> 4);
+              umma_f16(d_tmem, adesc + step, bdesc + step, idesc, (done_kb > 0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit(&empty[s]);
+            if (done_kb == total_kb - 1) umma_commit(&tfull[buf]);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (!ok && lane == 0) {
+      umma_commit(drain);
+      const long long start = clock64();
+      while (!mbar_try(drain, 0) && clock64() - start < 20000000LL) {}
+    }
+  } else if (warp >= 4) {
+    const int q = warp & 3;
+    const int c0 = ((warp - 4) >> 2) * 32;  // the 32 narrow columns this warp stores
+    const int cols = min(32, narrow - c0);
+    uint32_t tb = 0;
+    bool ok = true;
+    OutT* out = reinterpret_cast<OutT*>(p.out);
+    for (int t = 0; t < my_tiles && ok; ++t) {
+      const int g = tile_group(t), w = tile_column(t) + q * 32 + lane;
+      const bool has_rows = group_blocks(g) > 0;
+      uint32_t r[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = 0u;
+      if (has_rows) {
+        const int buf = tb & 1;
+        const uint32_t aph = (tb >> 1) & 1;
+        ++tb;
+        if (!mbar_wait_warp(&tfull[buf], aph, abort_flag, p.status, 54)) { ok = false; break; }
+        tc_fence_after_sync();
+        if (cols > 0) {
+          tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * kNarrowMax + c0, r);
+          tmem_ld_wait();
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[buf]);
+      }
+      if (w >= wide || cols <= 0) continue;
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+      if constexpr (TRANSPOSED) {
+        OutT* to = out + ((long long)g * p.M + c0) * p.N + w;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (j < cols) finish1<OutT>(to + (long long)j * p.N, v[j], p.scale, p.accumulate);
+      } else {
+        finish32<OutT>(out + ((long long)g * p.M + w) * p.N + c0, v, cols, p.scale, p.accumulate, p.wide_store != 0);
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 2) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, kNarrowTmemCols);
+  }
+}
+
+template <typename OutT>
+static int launch_narrow(const CUtensorMap& tg, const CUtensorMap& tx, const WgradParams& p, cudaStream_t s) {
+  const bool transposed = p.N > kNarrowMax;
+  const int wide = transposed ? p.N : p.M;
+  const int column_tiles = (wide + kWgBlockM - 1) / kWgBlockM;  // CTAs of a team; as many teams as fit
+  const int team_size = column_tiles < sm_count() ? column_tiles : sm_count();
+  const int teams = sm_count() / team_size < p.groups ? sm_count() / team_size : p.groups;
+  const int grid = team_size * teams;
+  auto kern = transposed ? grouped_wgrad_narrow_kernel<OutT, true> : grouped_wgrad_narrow_kernel<OutT, false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmemBytes) != cudaSuccess)
+    return B200MOE_ERR_LAUNCH;
+  kern<<<(unsigned)grid, kWgThreads, kNarrowSmemBytes, s>>>(transposed ? tx : tg, transposed ? tg : tx, p);
+  return launch_status();
+}
+
+// ---------------------------------------------------------------------------------------
 // CTA-pair variant: two CTAs of a cluster share one 256 x 256 output tile.  CTA r of the
 // pair owns output rows [r*128, r*128+128) (accumulated in its own TMEM) and loads, per K
 // block, its 128 columns of G and 128 of the 256 columns of X; one tcgen05.mma.cta_group::2
@@ -919,8 +1224,9 @@ static int grouped_wgrad_impl(const void* g, long long ldg, const void* x, long 
   p.g_scale = nullptr;
   p.x_scale = nullptr;
   p.wide_store = (((uintptr_t)out & 31) == 0 && ((size_t)N * esz) % 32 == 0 && ((size_t)M * N * esz) % 32 == 0) ? 1 : 0;
-  // Wide outputs go to the CTA-pair kernel (256-row tiles); narrow ones (LoRA factors) and the
-  // B200MOE_WGRAD_SINGLE=1 escape hatch use the single-CTA kernel.
+  // Wide outputs go to the CTA-pair kernel (256-row tiles), those with a side of at most 64 (LoRA
+  // factors) to the narrow one; what lies between, and everything under the B200MOE_WGRAD_SINGLE=1
+  // escape hatch, uses the single-CTA kernel.
   static const bool force_single = [] {
     const char* v = getenv("B200MOE_WGRAD_SINGLE");
     return v != nullptr && v[0] == '1';
@@ -928,6 +1234,8 @@ static int grouped_wgrad_impl(const void* g, long long ldg, const void* x, long 
   if (!force_single && M > 128 && N > 128) {
     return out_is_fp32 ? launch_pair<float>(tg, tx, p, s) : launch_pair<__nv_bfloat16>(tg, tx, p, s);
   }
+  if (!force_single && (M <= kNarrowMax || N <= kNarrowMax))
+    return out_is_fp32 ? launch_narrow<float>(tg, tx, p, s) : launch_narrow<__nv_bfloat16>(tg, tx, p, s);
   const long long tiles = (long long)groups * ((M + kWgBlockM - 1) / kWgBlockM) * ((N + kWgBlockN - 1) / kWgBlockN);
   long long grid = tiles < sm_count() ? tiles : sm_count();
   if (out_is_fp32) {

@@ -205,7 +205,34 @@ def test_wgrad(counts, m, n, out_dtype):
             assert mean <= (1e-6 if out_dtype == torch.float32 else MEAN_REL), mean
 
 
-@pytest.mark.parametrize("m,n", [(256, 512), (128, 256)])  # the CTA-pair kernel and the single-CTA kernel
+@pytest.mark.parametrize("m,n", [(8, 304), (304, 8), (64, 128), (200, 64), (40, 24), (16, 1032)])
+@pytest.mark.parametrize("counts", [[0, 70, 1300, 15, 0, 64, 1], [5], [0, 0, 3000, 129]])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_wgrad_with_one_narrow_side(counts, m, n, out_dtype):
+    """Either side at most 64 wide, groups from nothing to most of the rows (more and fewer tiles than
+    SMs), against float64; then the same added, times a scale, to a buffer."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(m + n)
+    rows, groups = sum(counts), len(counts)
+    left, right = torch.randn(rows, m, generator=g).bfloat16(), torch.randn(rows, n, generator=g).bfloat16()
+    offsets = _offsets(counts)
+    expected = torch.stack([left[lo:hi].double().t() @ right[lo:hi].double()
+                            for lo, hi in zip(offsets[:-1].tolist(), offsets[1:].tolist())])
+    got = ops.grouped_wgrad(left.to(DEV), right.to(DEV), offsets.to(DEV), groups, out_dtype)
+    ops.check_status(DEV)
+    # fp32 sums of up to 3000 products of magnitude 1 (2^-24 a step), one rounding to bf16 (8 significant bits: 2^-8)
+    bound = 2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0
+    slack = 3000 * 2.0 ** -24 * max(counts) ** 0.5
+    assert ((got.cpu().double() - expected).abs() <= bound * expected.abs() + slack).all()
+    assert (got[[i for i, c in enumerate(counts) if c == 0]] == 0).all()
+    start = torch.randn(groups, m, n, generator=g).to(out_dtype)
+    buffer = start.to(DEV)
+    ops.grouped_wgrad(left.to(DEV), right.to(DEV), offsets.to(DEV), groups, accumulate_into=buffer, scale=0.5)
+    total = start.double() + 0.5 * expected
+    assert ((buffer.cpu().double() - total).abs() <= (bound + 2.0 ** -23) * total.abs() + slack).all()
+
+
+@pytest.mark.parametrize("m,n", [(256, 512), (128, 256), (16, 256), (256, 16)])  # the CTA-pair, single-CTA, narrow kernels
 def test_wgrad_groups_are_isolated_from_a_neighbours_inf_and_nan(m, n):
     """The last K block of a group is loaded together with the first rows of the next group;
     both operand tiles are zeroed past the group's end, so an Inf or NaN there cannot reach
