@@ -529,6 +529,14 @@ typedef struct b200moe_backward_args {
 long long b200moe_backward_workspace_bytes(long long tokens, int width, int inner, int experts, int top_k);
 int b200moe_backward_fp8(const b200moe_backward_args* args, void* stream);
 
+/*
+ * dst[slots[t * fanout + k], :] = src[t, :] (bf16 rows of `width`): b200moe_gather_rows with
+ * gather = order, gather_div = fanout, from the token's side.  A slot outside [0, rows_out) is
+ * reported and skipped.  fanout <= 32.
+ */
+int b200moe_scatter_rows(const void* src, long long lds, long long tokens, const int32_t* slots, int fanout,
+                         long long rows_out, int width, void* dst, long long ldd, int32_t* status, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

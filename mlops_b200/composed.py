@@ -96,7 +96,7 @@ def prepare_bwd(grad_aux: torch.Tensor, grad_probability_sum: torch.Tensor, grad
         gh = grad_h13.contiguous()
         gh_q, gh_s = ops.quantize_rows(gh)  # the bf16 gradient that crossed the regions, as E4M3
         if need_w13:
-            x_rows = ops.dispatch(flat, order, int(top_k))
+            x_rows = layer.expert_rows(flat, order, slots, int(top_k))
             grad_w13 = ops.grouped_wgrad(gh, x_rows, offsets, experts, wdtype)
             del x_rows
         else:

@@ -162,7 +162,7 @@ extern "C" int b200moe_backward_fp8(const b200moe_backward_args* a, void* stream
     B200_STEP(b200moe_grouped_wgrad_bf16(a->rows, D, a->r, F, a->offsets, E, 1, R, D, F, a->grad_w2,
                                          a->weight_gradients_fp32, a->status, stream));
   if (a->grad_w13 != nullptr) {
-    B200_STEP(b200moe_gather_rows(a->x, D, T, a->order, K, R, D, a->rows, D, a->status, stream));
+    B200_STEP(b200moe_scatter_rows(a->x, D, T, a->slots, K, R, D, a->rows, D, a->status, stream));
     B200_STEP(b200moe_grouped_wgrad_bf16(a->gh, 2LL * F, a->rows, D, a->offsets, E, 1, R, 2 * F, D, a->grad_w13,
                                          a->weight_gradients_fp32, a->status, stream));
   }

@@ -196,7 +196,7 @@ def forward_routed(
         if bf16_weights:
             # the bf16 compute path (reference: src/mlops/kernels/moe_grouped_gemm.py:201-299 around
             # the builtin's dispatch / SwiGLU / combine): nothing is quantised
-            x_rows = ops.dispatch(h2_flat, order, int(top_k))
+            x_rows = expert_rows(h2_flat, order, slots, int(top_k))
             h13 = ops.grouped_gemm_bf16(x_rows, w13_data, offsets)
             del x_rows
             _q, _s, act = ops.swiglu_quantize(h13, limit=swiglu_limit, quantized=False, rounded=True)
@@ -225,6 +225,14 @@ def forward_routed(
             logits, route_ids, counts, routing_mode=str(routing_mode), lengths=normalized, experts=experts
         )
     return (output, aux, counts, probability_sum, logits, route_weights, route_ids, order, offsets, slots, h13)
+
+
+def expert_rows(x, order, slots, top_k):
+    """bf16 rows of `x [T, D]` in expert order, from the token's side where `slots` is the sort's
+    `[T, K]` (each row is then read once for its copies), else gathered by `order`."""
+    if top_k <= 32 and ops.dense(slots, torch.int32, x.shape[0], top_k):
+        return ops.scatter_rows(x, slots)
+    return ops.dispatch(x, order, top_k)
 
 
 def _one_sequence(routing_mode, lengths):
@@ -325,7 +333,7 @@ def backward_routed(
         counts = (offsets[1:] - offsets[:-1]).long()
 
         if bf16_weights:
-            dy_rows = ops.dispatch(grad_flat, order, int(top_k))
+            dy_rows = expert_rows(grad_flat, order, slots, int(top_k))
             r = ops.grouped_gemm_bf16(dy_rows, w2_data, offsets, b_mn_major=True)
             dscore, _gq, _gs, gh_b, act_scaled = ops.dswiglu_routed(
                 h13, r, route_weights, order, limit=swiglu_limit, quantized=False, rounded=True,
@@ -340,7 +348,7 @@ def backward_routed(
                 grad_w2 = torch.empty(0, dtype=wdtype, device=h2.device)
             del dy_rows
             if need_w13:
-                x_rows = ops.dispatch(h2_flat, order, int(top_k))
+                x_rows = expert_rows(h2_flat, order, slots, int(top_k))
                 grad_w13 = _weight_gradient(gh_b, x_rows, offsets, experts, wdtype, weight_grad_operands)
                 del x_rows
             else:
@@ -370,7 +378,7 @@ def backward_routed(
         else:
             grad_w2 = torch.empty(0, dtype=wdtype, device=h2.device)
         if need_w13:
-            x_rows = ops.dispatch(h2_flat, order, int(top_k))
+            x_rows = expert_rows(h2_flat, order, slots, int(top_k))
             grad_w13 = _weight_gradient(gh_b, x_rows, offsets, experts, wdtype, weight_grad_operands)
             del x_rows, gh_b
         else:

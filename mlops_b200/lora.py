@@ -144,7 +144,7 @@ def _lora_backward(grad_output, grad_aux, grad_probability_sum, hidden, router_w
             h13, r, weights, order, limit=swiglu_limit, quantized=True, rounded=True, scaled_activation=True)
         grad_route_weights = ops.gather_scalar(dscore, slots)
 
-        x_rows = ops.dispatch(flat, order, top_k)
+        x_rows = layer.expert_rows(flat, order, slots, int(top_k))
         dt1 = ops.lora_project(gh_b, b13t, offsets, rank_major=True)                # gh B13     [R, r]
         fdtype = a13.dtype
         grad_a13 = grad_b13 = grad_a2 = grad_b2 = empty(fdtype)

@@ -886,6 +886,28 @@ def dispatch(x, order, top_k):
 
 
 @_on_tensor_device
+def scatter_rows(x, slots):
+    """`dispatch(x, order, K)` from the token's side: every bf16 row of `x [T, D]` written to the K rows
+    `slots[t, :]` (the sort's inverse permutation, int32 `[T, K]`, K at most 32)."""
+    device = _need_cuda(x, slots)
+    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1:
+        raise NativeError("x must be bf16 [rows, width] with unit inner stride")
+    if slots.dtype != torch.int32 or slots.dim() != 2 or slots.shape[0] != x.shape[0] or not slots.is_contiguous():
+        raise NativeError("slots must be contiguous int32 [rows of x, fan-out]")
+    tokens, fanout = slots.shape
+    out = torch.empty((tokens * fanout, x.shape[1]), dtype=torch.bfloat16, device=device)
+    if out.shape[0] == 0:
+        return out
+    check(
+        lib.b200moe_scatter_rows(x.data_ptr(), x.stride(0), tokens, slots.data_ptr(), fanout, out.shape[0], x.shape[1],
+                                 out.data_ptr(), out.stride(0), status_block(device).data_ptr(), _stream()),
+        "scatter_rows",
+    )
+    _count()
+    return out
+
+
+@_on_tensor_device
 def gather_scalar(values, slots):
     """`values[slots]` (fp32), shaped like `slots`."""
     _need_cuda(values, slots)

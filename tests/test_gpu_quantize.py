@@ -260,6 +260,8 @@ def test_row_kernels_at_the_edges_of_their_pieces(tokens, width, top_k):
     q, s, copy = ops.quantize_rows_scatter(x.to(DEV), slots.to(DEV), with_copy=True)
     assert torch.equal(q.cpu().view(U8), q_ref.view(U8)) and torch.equal(s.cpu(), s_ref)
     assert torch.equal(copy.cpu(), rows) and torch.equal(ops.dispatch(x.to(DEV), order.to(DEV), top_k).cpu(), rows)
+    if top_k <= 32:
+        assert torch.equal(ops.scatter_rows(x.to(DEV), slots.to(DEV)).cpu(), rows)
     weights = torch.randint(-3, 2, (tokens, top_k), generator=g).float().exp2()  # products are exact, fused or not
     residual = torch.randn(tokens, width, generator=g).bfloat16()
     got = ops.combine(rows.to(DEV), slots.to(DEV), weights.to(DEV), residual.to(DEV))
