@@ -29,6 +29,11 @@ EncodeTiledFn get_encode_tiled();
 // Rows of tiles a GEMM walks together (banded_tile): `bytes` is what one row of tiles reads of the
 // operand that runs along it (a group's whole weight, or its rows of X in a weight gradient).
 int tile_band(long long bytes);
+// b200moe_routing_probability_sum and, with counts (the sort's, int64) and aux, the auxiliary loss of
+// the rows as one sequence.
+int launch_routing_statistics(const float* logits, long long ld, long long tokens, int experts, int mode,
+                              void* workspace, float* probability_sum, const long long* counts, int top_k, float* aux,
+                              cudaStream_t s);
 // b200moe_routing_gradient, with the gradient written as two bf16 pieces [tokens, experts] as well
 // (high + low; both or neither).
 int launch_routing_gradient(const float* logits, long long ld, long long tokens, int experts, int top_k, int mode,

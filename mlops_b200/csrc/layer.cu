@@ -13,29 +13,6 @@
 
 namespace b200 {
 
-// Auxiliary loss of one sequence from the probability sum and the sort's counts, one block:
-// softmax modes  experts * sum_e (counts_e / assignments) * (psum_e / tokens)
-// sigmoid mode   sum_e (counts_e * experts / assignments) * (psum_e / tokens)
-__global__ void __launch_bounds__(1024)
-auxiliary_loss_kernel(const float* __restrict__ psum, const long long* __restrict__ counts, int experts,
-                      float assignments, float tokens, int sigmoid, float* __restrict__ aux) {
-  __shared__ float sums[32];
-  const int e = threadIdx.x;
-  float v = 0.f;
-  if (e < experts) {
-    const float count = (float)counts[e];
-    const float frequency = sigmoid ? __fdiv_rn(count * (float)experts, assignments) : __fdiv_rn(count, assignments);
-    v = frequency * __fdiv_rn(psum[e], tokens);
-  }
-  v = warp_sum(v);
-  if ((e & 31) == 0) sums[e >> 5] = v;
-  __syncthreads();
-  if (e < 32) {
-    v = warp_sum(e < (int)(blockDim.x >> 5) ? sums[e] : 0.f);
-    if (e == 0) *aux = sigmoid ? v : (float)experts * v;
-  }
-}
-
 // The frequencies the auxiliary loss's gradient needs, from the sort's offsets.
 __global__ void frequency_kernel(const int* __restrict__ offsets, int experts, float assignments, int sigmoid,
                                  float* __restrict__ frequency) {
@@ -128,10 +105,8 @@ extern "C" int b200moe_forward_fp8(const b200moe_forward_args* a, void* stream) 
                                      a->offsets, E, E, R, D, F, 0, 256, a->status, stream));
   B200_STEP(b200moe_combine(a->expert_rows, D, R, a->slots, a->route_weights, a->residual, D, a->output, D, T, D, K,
                             stream));
-  B200_STEP(b200moe_routing_probability_sum(a->logits, E, T, E, a->mode, s.statistics, a->probability_sum, stream));
-  auxiliary_loss_kernel<<<1, (E + 31) / 32 * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      a->probability_sum, a->counts, E, (float)R, (float)T, a->mode == B200MOE_ROUTE_SIGMOID_NOAUX_TC, a->aux);
-  return launch_status();
+  return launch_routing_statistics(a->logits, E, T, E, a->mode, s.statistics, a->probability_sum, a->counts, K, a->aux,
+                                   reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" long long b200moe_backward_workspace_bytes(long long tokens, int width, int inner, int experts, int top_k) {

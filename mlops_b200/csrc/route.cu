@@ -16,7 +16,8 @@
 //   order[j]   flat assignment index (token*K + slot) held by sorted row j
 //   offsets[e] first sorted row of expert e (offsets[E] = T*K)
 //   slots[i]   sorted row of flat assignment i (the inverse permutation)
-// Three launches: per-chunk histogram, scan (over chunks, then experts), ranked scatter.
+// Three launches: per-chunk histogram, scan (over chunks, then experts), ranked scatter; one for a
+// single chunk.
 #include "common.cuh"
 #include "host_util.h"
 
@@ -318,6 +319,72 @@ sort_scatter_kernel(const int* __restrict__ ids, int R, int E, const int* __rest
   }
 }
 
+// The whole sort of up to kSortChunk assignments in one block: the counts per warp and expert of the
+// scatter pass also give the histogram, so its scan and the ranks need no other launch.  (Three
+// launches: 8.2 us of kernels for 8 assignments, 12 for 1024 of 8 experts, 13.5 for 512 of 256; this takes
+// 3.3, 3.7 and 4.1.)
+__global__ void __launch_bounds__(kSortThreads)
+sort_small_kernel(const int* __restrict__ ids, int R, int E, int* __restrict__ offsets, long long* __restrict__ counts64,
+                  int* __restrict__ order, int* __restrict__ slots, int* status) {
+  extern __shared__ int cnt[];  // [kSortWarps][E]
+  __shared__ int warp_tot[kSortWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < kSortWarps * E; i += kSortThreads) cnt[i] = 0;
+  __syncthreads();
+  const int per_warp = ((R + kSortWarps - 1) / kSortWarps + 31) / 32 * 32;
+  const int begin = warp * per_warp, end = min(R, begin + per_warp);
+  int* mine = cnt + warp * E;
+  for (int i = begin + lane; i < end; i += 32) {
+    const int e = ids[i];
+    if (e < 0 || e >= E) report_error(status, ERR_BAD_OFFSETS, 10, i);
+    atomicAdd(&mine[clamp_id(e, E)], 1);
+  }
+  __syncthreads();
+  // thread i scans experts [i * per_thread, (i + 1) * per_thread)
+  const int per_thread = (E + kSortThreads - 1) / kSortThreads;
+  const int e_begin = threadIdx.x * per_thread, e_end = min(E, e_begin + per_thread);
+  int total = 0;
+  for (int e = e_begin; e < e_end; ++e)
+    for (int w = 0; w < kSortWarps; ++w) total += cnt[w * E + e];
+  int incl = total;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  int base = incl - total;
+  for (int w = 0; w < warp; ++w) base += warp_tot[w];
+  for (int e = e_begin; e < e_end; ++e) {
+    offsets[e] = base;
+    const int first = base;
+    for (int w = 0; w < kSortWarps; ++w) {
+      const int v = cnt[w * E + e];
+      cnt[w * E + e] = base;
+      base += v;
+    }
+    if (counts64 != nullptr) counts64[e] = base - first;
+  }
+  if (threadIdx.x == 0) offsets[E] = R;
+  __syncthreads();
+  for (int i0 = begin; i0 < end; i0 += 32) {
+    const int i = i0 + lane;
+    const int e = i < end ? clamp_id(ids[i], E) : -1;
+    const uint32_t peers = __match_any_sync(0xffffffffu, e);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    int pos = 0;
+    if (e >= 0) pos = mine[e] + rank;
+    __syncwarp();
+    if (e >= 0 && rank == 0) mine[e] += __popc(peers);
+    __syncwarp();
+    if (e >= 0) {
+      order[pos] = i;
+      slots[i] = pos;
+    }
+  }
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -378,6 +445,11 @@ static int launch_sort(const int32_t* ids, int R, int experts, int32_t* order, i
                        int32_t* slots, long long* counts64, int* chunk_hist, int32_t* status,
                        cudaStream_t s) {
   const int nchunks = (R + kSortChunk - 1) / kSortChunk;
+  if (nchunks == 1) {
+    sort_small_kernel<<<1, kSortThreads, kSortWarps * experts * 4, s>>>(ids, R, experts, offsets, counts64, order,
+                                                                       slots, status);
+    return launch_status();
+  }
   if (nchunks > 0) {
     sort_hist_kernel<<<nchunks, kSortThreads, experts * 4, s>>>(ids, R, experts, chunk_hist, status);
   }

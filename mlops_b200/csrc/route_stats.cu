@@ -92,13 +92,34 @@ probability_partials_kernel(const float* __restrict__ logits, long long ld, long
   }
 }
 
-__global__ void probability_finish_kernel(const float* __restrict__ partials, int blocks, int E,
-                                          float* __restrict__ psum) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
+// One block, a thread per expert.  With `counts` also the auxiliary loss of one sequence:
+//   softmax modes  experts * sum_e (counts_e / assignments) * (psum_e / tokens)
+//   sigmoid mode   sum_e (counts_e * experts / assignments) * (psum_e / tokens)
+__global__ void __launch_bounds__(1024)
+probability_finish_kernel(const float* __restrict__ partials, int blocks, int E, float* __restrict__ psum,
+                          const long long* __restrict__ counts, float assignments, float tokens, int sigmoid,
+                          float* __restrict__ aux) {
+  __shared__ float sums[32];
+  const int e = threadIdx.x;
   float v = 0.f;
-  for (int b = 0; b < blocks; ++b) v += partials[(long long)b * E + e];  // blocks in order
-  psum[e] = v;
+  if (e < E) {
+#pragma unroll 8
+    for (int b = 0; b < blocks; ++b) v += partials[(long long)b * E + e];  // blocks in order
+    psum[e] = v;
+  }
+  if (counts == nullptr) return;
+  if (e < E) {
+    const float count = (float)counts[e];
+    const float frequency = sigmoid ? __fdiv_rn(count * (float)E, assignments) : __fdiv_rn(count, assignments);
+    v = frequency * __fdiv_rn(v, tokens);
+  }
+  v = warp_sum(v);
+  if ((e & 31) == 0) sums[e >> 5] = v;
+  __syncthreads();
+  if (e < 32) {
+    v = warp_sum(e < (int)(blockDim.x >> 5) ? sums[e] : 0.f);
+    if (e == 0) *aux = sigmoid ? v : (float)E * v;
+  }
 }
 
 template <int EPL>
@@ -239,7 +260,13 @@ extern "C" int b200moe_routing_probability_sum(const float* logits, long long ld
   if (!logits || !workspace || !probability_sum || tokens < 0 || experts <= 0 || mode < 0 || mode > 2)
     return B200MOE_ERR_ARG;
   if (experts > 1024) return B200MOE_ERR_LIMIT;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return launch_routing_statistics(logits, ld, tokens, experts, mode, workspace, probability_sum, nullptr, 1, nullptr,
+                                   reinterpret_cast<cudaStream_t>(stream));
+}
+
+int b200::launch_routing_statistics(const float* logits, long long ld, long long tokens, int experts, int mode,
+                                    void* workspace, float* probability_sum, const long long* counts, int top_k,
+                                    float* aux, cudaStream_t s) {
   const long long blocks = stat_blocks(tokens);
   const long long per_block = (tokens + blocks - 1) / blocks;
   float* partials = reinterpret_cast<float*>(workspace);
@@ -248,7 +275,9 @@ extern "C" int b200moe_routing_probability_sum(const float* logits, long long ld
       logits, ld, tokens, experts, mode, per_block, partials)
   B200_DISPATCH_EPL(experts, CALL_PARTIALS);
 #undef CALL_PARTIALS
-  probability_finish_kernel<<<(experts + 255) / 256, 256, 0, s>>>(partials, (int)blocks, experts, probability_sum);
+  probability_finish_kernel<<<1, (experts + 31) / 32 * 32, 0, s>>>(partials, (int)blocks, experts, probability_sum,
+                                                                   counts, (float)(tokens * top_k), (float)tokens,
+                                                                   mode == 2, aux);
   return launch_status();
 }
 

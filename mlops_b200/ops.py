@@ -251,7 +251,7 @@ def sort_assignments(route_ids, experts):
         ),
         "sort_assignments",
     )
-    _count(3 if n > 0 else 1)
+    _count(3 if n > 4096 else 1)
     return order, offsets, slots.view(route_ids.shape), counts
 
 
@@ -273,7 +273,7 @@ def sort_assignments_static(route_ids, experts, order, offsets, slots, counts):
         ),
         "sort_assignments_static",
     )
-    _count(3 if route_ids.numel() > 0 else 1)
+    _count(3 if route_ids.numel() > 4096 else 1)
 
 
 # ------------------------------------------------------------------------ quantisation
@@ -975,7 +975,7 @@ def forward_fp8(x, residual, logits, w13, w2, *, top_k, mode, bias=None, n_group
         h13.data_ptr(), output.data_ptr(), aux.data_ptr(), probability_sum.data_ptr(), x_q.data_ptr(),
         act_q.data_ptr(), expert_rows.data_ptr(), workspace.data_ptr(), status_block(device).data_ptr())
     check(lib.b200moe_forward_fp8(ctypes.byref(args), _stream()), "forward_fp8")
-    _count(12)
+    _count(11 if rows > 4096 else 9)
     return output, aux, counts, probability_sum, weights, ids, order, offsets, slots, h13
 
 

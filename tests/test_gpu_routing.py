@@ -61,6 +61,29 @@ def test_route_ids_bit_exact_on_seeded_logits(tokens, experts, top_k, mode, n_gr
     torch.testing.assert_close(w.cpu(), w_ref, rtol=2e-6, atol=1e-7)
 
 
+@pytest.mark.parametrize("assignments", [1, 31, 257, 4095, 4096, 4097, 8192])
+@pytest.mark.parametrize("experts", [1, 9, 257, 1024])
+def test_sort_of_one_chunk_and_of_several(assignments, experts):
+    """Up to 4096 assignments are sorted by one block, more by three launches; ids out of range are
+    reported and sorted as the nearest expert by both."""
+    from mlops_b200._lib import NativeError
+
+    ops = _ops()
+    g = torch.Generator().manual_seed(assignments + experts)
+    ids = torch.randint(0, experts, (assignments, 1), generator=g).to(torch.int32)
+    order, offsets, slots, counts = ops.sort_assignments(ids.to(DEV), experts)
+    o_ref, f_ref, s_ref = O.sort_assignments(ids, experts)
+    assert torch.equal(order.cpu(), o_ref) and torch.equal(offsets.cpu(), f_ref) and torch.equal(slots.cpu(), s_ref)
+    assert torch.equal(counts.cpu(), torch.bincount(ids.view(-1).long(), minlength=experts))
+    ops.check_status(DEV)
+    ids[-1], ids[0] = experts + 3, -7 if assignments > 1 else experts + 3
+    order, offsets, _slots, _counts = ops.sort_assignments(ids.to(DEV), experts)
+    o_ref, f_ref, _ = O.sort_assignments(ids.clamp(0, experts - 1), experts)
+    assert torch.equal(order.cpu(), o_ref) and torch.equal(offsets.cpu(), f_ref)
+    with pytest.raises(NativeError):
+        ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("experts,top_k,n_group,topk_group", [(1, 1, 1, 1), (33, 5, 3, 2), (64, 6, 32, 5), (256, 8, 8, 4),
                                                               (1024, 32, 32, 31), (40, 3, 40, 40), (12, 2, 12, 3)])
 @pytest.mark.parametrize("mode", ["softmax_then_topk", "topk_then_softmax", "sigmoid_noaux_tc"])
