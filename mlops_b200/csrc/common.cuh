@@ -469,60 +469,32 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float scale) {
   return make_uint2(w[0], w[1]);
 }
 
-// sigmoid(g) = 1 / (1 + exp(-g)) of two values with |g| < kSigmoidFast.  exp(-g) = 2^n (1 + t): with
-// BF16 (g has 8 significant bits) n is g times the upper 16 bits of -log2(e), an exact product, and t
-// = -g ln(2) times the rest, below 6e-5; otherwise n is the rounded product and t its remainder by
-// fma.  With e = 2^n from the special-function unit and y the hardware's reciprocal of d = 1 + e
-// rounded, what d lost and e t enter with the residual of the Newton step: y + y (1 - d y - c y).
-// Some 13 packed or special-function instructions for two values, against some forty of two expf and
-// two rounded divisions, which made the SwiGLU kernels issue-bound.  Relative error against 64 bits,
-// largest / rms, for |g| below 12: bf16 values 1.33e-7 / 1.43e-8 (the library functions 1.33e-7 /
-// 1.93e-8), any values 1.69e-7 / 3.8e-8 (1.74e-7 / 4.2e-8).  Above, the largest errors would be larger.
-constexpr float kSigmoidFast = 12.0f;
-template <bool BF16>
-__device__ __forceinline__ void sigmoid2(float g0, float g1, float& s0, float& s1) {
-  constexpr double kLog2E = 1.4426950408889634074, kLn2 = 0.69314718055994530942;
-  const Float2 one = splat2(1.0f), minus_one = splat2(-1.0f);
-  const Float2 g = pack2(g0, g1);
-  Float2 n, minus_t;
-  if constexpr (BF16) {
-    constexpr float kHigh = (float)((double)(int)(kLog2E * 32768.0) / 32768.0);
-    n = mul2(g, splat2(-kHigh));
-    minus_t = mul2(g, splat2((float)((kLog2E - (double)kHigh) * kLn2)));
-  } else {
-    constexpr float kHigh = (float)kLog2E, kLow = (float)(kLog2E - (double)kHigh);
-    n = mul2(g, splat2(-kHigh));
-    minus_t = mul2(mad2(g, splat2(kLow), mad2(g, splat2(kHigh), n)), splat2((float)kLn2));
-  }
-  float n0, n1, e0, e1;
-  unpack2(n, n0, n1);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(n0));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(n1));
-  const Float2 e = pack2(e0, e1);
-  const Float2 minus_d = mad2(e, minus_one, minus_one);
-  const Float2 lost = mad2(e, minus_one, mad2(minus_d, minus_one, minus_one));  // (d - 1) - e
-  const Float2 minus_c = mad2(e, minus_t, lost);
-  float d0, d1, y0, y1;
-  unpack2(minus_d, d0, d1);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(-d0));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(-d1));
-  const Float2 y = pack2(y0, y1);
-  const Float2 residual = mad2(minus_c, y, mad2(minus_d, y, one));
-  unpack2(mad2(y, residual, y), s0, s1);
-}
-// ... of any eight values: those outside the range, infinities and NaN take the library functions.
-// A value's result does not depend on its neighbours.
-template <bool BF16>
+// sigmoid(g) = 1 / (1 + exp(-g)) of eight values: the library's exponential and a reciprocal rounded
+// to nearest.  d = 1 + exp(-g) lies in [1, 2^126) from g = -80 on; there the hardware's reciprocal y
+// (within one ulp) and one Newton step, y + y (1 - d y) by two fma's, give the rounded reciprocal for
+// every d whose significand is not all ones (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990, theorem 7) and, tried with all 2^23 significands, for that
+// one as well.  Two values at a time with packed instructions; __frcp_rn, which serves the rest
+// of the range, made the SwiGLU kernels issue-bound.  A value's result does not depend on its neighbours.
+constexpr float kSigmoidFast = -80.0f;
 __device__ __forceinline__ void sigmoid8(const float (&g)[8], float (&s)[8]) {
-  float top = 0.f;
+  const Float2 one = splat2(1.0f), minus_one = splat2(-1.0f);
+  float low = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) top = fmaxf(top, fabsf(g[i]));  // (a NaN stays a NaN either way)
-#pragma unroll
-  for (int i = 0; i < 8; i += 2) sigmoid2<BF16>(g[i], g[i + 1], s[i], s[i + 1]);
-  if (!(top < kSigmoidFast)) {
+  for (int i = 0; i < 8; i += 2) {
+    low = fminf(low, fminf(g[i], g[i + 1]));  // (a NaN stays a NaN either way)
+    const Float2 minus_d = mad2(pack2(expf(-g[i]), expf(-g[i + 1])), minus_one, minus_one);
+    float d0, d1, y0, y1;
+    unpack2(minus_d, d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(-d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(-d1));
+    const Float2 y = pack2(y0, y1);
+    unpack2(mad2(y, mad2(minus_d, y, one), y), s[i], s[i + 1]);
+  }
+  if (low < kSigmoidFast) {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (!(fabsf(g[i]) < kSigmoidFast)) s[i] = __frcp_rn(1.0f + expf(-g[i]));
+      if (g[i] < kSigmoidFast) s[i] = __frcp_rn(1.0f + expf(-g[i]));
   }
 }
 

@@ -1064,8 +1064,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 u8[i] = fminf(fmaxf(u8[i], -p.limit), p.limit);
               }
             }
-            if (p.limited) sigmoid8<false>(g8, sig);
-            else sigmoid8<true>(g8, sig);
+            sigmoid8(g8, sig);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               acc[j + i] = g8[i] * sig[i] * u8[i];

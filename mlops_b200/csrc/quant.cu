@@ -164,9 +164,9 @@ quantize_scatter_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, long
 // once: to E4M3 with 1x128 scales (act_q / scales) and, when act_bf16 is given, to bf16.
 // Optional GLM clamp: gate capped at `limit`, up clipped to [-limit, limit].
 // One warp per `per_warp` consecutive pieces of 256 columns of a row: the next piece is loaded
-// while one is worked on.  Issue-bound in its arithmetic: 45 instructions a value with the library's
-// exponential and division; with sigmoid8 and packed arithmetic 32768 rows of F = 14336 take 0.46 ms
-// (5.1 TB/s) instead of 0.61, 512 rows of F = 2048 take 4.1 us instead of 10.
+// while one is worked on.  Issue-bound in its arithmetic: with the library's rounded reciprocal and scalar
+// arithmetic 32768 rows of F = 14336 took 0.61 ms, with sigmoid8 and packed arithmetic 0.475 (5.0 TB/s);
+// 512 rows of F = 2048 take 4.1 us instead of 10.
 template <bool LIMITED>
 __global__ void __launch_bounds__(kRowWarps * 32)
 swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h13, long long ldh, long long rows, int F,
@@ -201,7 +201,7 @@ swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h13, long long ldh, long l
         u[i] = fminf(fmaxf(u[i], -limit), limit);
       }
     }
-    sigmoid8<!LIMITED>(g, sig);  // a limit may have more significant bits than bf16
+    sigmoid8(g, sig);
     float amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
@@ -233,10 +233,12 @@ swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h13, long long ldh, long l
 // the sixteen h13 values of an iteration before it stores the sixteen gradients to the same
 // addresses, and no other thread touches them; act_scaled may alias r in the same way.
 // One warp per row (the dot product stays in the warp); the next 256 columns are loaded while
-// these are worked on.  32768 rows of F = 14336 with every output: 1.09 ms (6.0 TB/s); 1.36 ms with
-// 77 scalar instructions a value, which kept the kernel issue-bound.
+// these are worked on.  32768 rows of F = 14336 with every output: 1.10 ms (6.0 TB/s); 1.36 ms with
+// scalar arithmetic, which kept the kernel issue-bound.  Three blocks to an SM need 80 registers a
+// thread; at the 83 the compiler takes unasked two fit, and the same took 1.20 ms.  (With a limit 80
+// would spill.)
 template <bool LIMITED>
-__global__ void __launch_bounds__(kRowWarps * 32)
+__global__ void __launch_bounds__(kRowWarps * 32, LIMITED ? 2 : 3)
 dswiglu_routed_kernel(const __nv_bfloat16* h13, long long ldh,  // may be the same buffer as gh_bf16
                       const __nv_bfloat16* rmat, long long ldr,       // may be the same buffer as act_scaled
                       const float* __restrict__ route_weights, long long n_weights,
@@ -267,10 +269,11 @@ dswiglu_routed_kernel(const __nv_bfloat16* h13, long long ldh,  // may be the sa
   }
   const Float2 score = splat2(route_weights[which]);
   const Float2 one = splat2(1.0f), minus_one = splat2(-1.0f);
-  Float2 dot2 = splat2(0.f);
+  float dot = 0.f;
   for (int c0 = 0; c0 < F; c0 += 256) {
     const int c = c0 + lane * 8;
-    float g[8], u[8], rv[8], dg[8], du[8], as[8], sig[8];
+    float g[8], u[8], rv[8], dg[8], du[8], sig[8];
+    uint32_t scaled[4];  // score * act
     unpack8(rg, g);
     unpack8(ru, u);
     unpack8(rx, rv);
@@ -285,19 +288,22 @@ dswiglu_routed_kernel(const __nv_bfloat16* h13, long long ldh,  // may be the sa
         u[i] = fminf(fmaxf(u[i], -limit), limit);
       }
     }
-    sigmoid8<!LIMITED>(g, sig);
+    sigmoid8(g, sig);
     float amax_g = 0.f, amax_u = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
       const Float2 s2 = pack2(sig[i], sig[i + 1]), u2 = pack2(u[i], u[i + 1]), r2 = pack2(rv[i], rv[i + 1]);
       const Float2 silu = mul2(pack2(g[i], g[i + 1]), s2);
       const Float2 act = mul2(silu, u2);
-      dot2 = mad2(r2, act, dot2);
+      float act0, act1;
+      unpack2(act, act0, act1);
+      dot = fmaf(rv[i + 1], act1, fmaf(rv[i], act0, dot));  // one sum in column order
       const Float2 go = mul2(score, r2);
       const Float2 slope = mad2(silu, mad2(s2, minus_one, one), s2);  // sig + silu (1 - sig)
       unpack2(mul2(mul2(go, u2), slope), dg[i], dg[i + 1]);
       unpack2(mul2(go, silu), du[i], du[i + 1]);
-      unpack2(mul2(score, act), as[i], as[i + 1]);
+      unpack2(mul2(score, act), act0, act1);
+      scaled[i / 2] = pack_bf16x2(act0, act1);
       if constexpr (LIMITED) {
 #pragma unroll
         for (int h = i; h < i + 2; ++h) {
@@ -325,12 +331,11 @@ dswiglu_routed_kernel(const __nv_bfloat16* h13, long long ldh,  // may be the sa
         *reinterpret_cast<uint4*>(gh_bf16 + r * ldg + c) = pack8_bf16(dg);
         *reinterpret_cast<uint4*>(gh_bf16 + r * ldg + F + c) = pack8_bf16(du);
       }
-      if (act_scaled != nullptr) *reinterpret_cast<uint4*>(act_scaled + r * lda + c) = pack8_bf16(as);
+      if (act_scaled != nullptr)
+        *reinterpret_cast<uint4*>(act_scaled + r * lda + c) = make_uint4(scaled[0], scaled[1], scaled[2], scaled[3]);
     }
   }
-  float dot, odd;
-  unpack2(dot2, dot, odd);
-  dot = warp_sum(dot + odd);
+  dot = warp_sum(dot);
   if (lane == 0 && dscore != nullptr) dscore[r] = dot;
 }
 

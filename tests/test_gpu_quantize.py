@@ -222,7 +222,7 @@ def test_scatter_quantiser_equals_the_gathered_quantiser_bit_for_bit():
 def test_swiglu_over_the_whole_range_of_gates(rows, width, limit):
     """Gates from 2^-20 to 2^100, infinities and NaN: fp32 SwiGLU rounded once to bf16 is the float64
     value to one bf16 rounding (2^-8 relative, and 2^-20 of slack for the fp32 steps), values of the
-    two forms (library functions from |g| = 12 on) alike; a NaN stays one."""
+    two forms of the reciprocal (changing at g = -80) alike; a NaN stays one."""
     ops = _ops()
     g = torch.Generator().manual_seed(rows + width)
     gate = torch.randn(rows, width, generator=g) * torch.rand(rows, width, generator=g).mul(12).sub(6).exp2()
@@ -241,6 +241,32 @@ def test_swiglu_over_the_whole_range_of_gates(rows, width, limit):
     assert (error <= expected.abs()[~odd] * (2.0 ** -8 + 2.0 ** -20) + 1e-37).all()
     if limit is None:
         assert actual[0, 2].isnan() and actual[0, 0].isinf() and actual[0, 1].isnan()
+
+
+@pytest.mark.parametrize("limit", [None, 1.3])
+def test_swiglu_holds_the_library_functions_in_fp32(limit):
+    """silu of every finite bf16 gate in fp32, seen through the route-weight gradient (a one-hot r and up
+    = 1 make it silu itself): the bits of `g * reciprocal(1 + exp(-g))`, and within 7 x 2^-24 of the float64
+    value (exponential two ulp of 2^-23, sum, reciprocal and product half an ulp each)."""
+    ops = _ops()
+    gates = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    gates = gates[gates.isfinite()].view(-1, 8)  # eight consecutive patterns a row: neighbours in one thread
+    rows = gates.shape[0]
+    h13 = torch.cat([gates, torch.ones_like(gates)], dim=1).to(DEV)
+    order, ones = torch.arange(rows, dtype=torch.int32, device=DEV), torch.ones(rows, device=DEV)
+    g = gates.to(DEV).float()
+    if limit is not None:
+        g = g.clamp(max=limit)
+    same = g * torch.reciprocal(1.0 + torch.exp(-g))
+    exact = g.double() * torch.sigmoid(g.double())
+    for column in range(8):
+        r = torch.zeros(rows, 8, dtype=torch.bfloat16, device=DEV)
+        r[:, column] = 1.0
+        dscore = ops.dswiglu_routed(h13, r, ones, order, limit=limit, quantized=False, rounded=True)[0]
+        assert torch.equal(dscore, same[:, column])
+        normal = exact[:, column].abs() > 2.0 ** -120
+        error = (dscore.double() - exact[:, column]).abs()[normal]
+        assert (error <= 7 * 2.0 ** -24 * exact[:, column].abs()[normal]).all()
 
 
 @pytest.mark.parametrize("tokens,width,top_k", [(1, 8, 1), (3, 1032, 2), (70, 2048, 3), (5, 7168, 8), (9, 264, 11)])
