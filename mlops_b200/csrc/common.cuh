@@ -108,8 +108,8 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // One arrival on the mbarrier at the same shared-memory offset in CTA `cta` of the cluster.
-// This form orders the arrival after the thread's earlier accesses at CTA scope only: enough
-// when what the waiter consumes was written by the async proxy (TMA) or sits in TMEM.
+// This form orders the arrival after the thread's earlier accesses at CTA scope only: for what was
+// written by the async proxy (TMA) or sits in TMEM, never for ordinary stores.
 __device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t cta) {
   asm volatile(
       "{\n\t.reg .b32 remote;\n\t"
@@ -119,9 +119,10 @@ __device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t cta) 
       : "memory");
 }
 
-// The same arrival with release semantics at cluster scope: the waiter in the other CTA may
-// consume what this thread (and, through the fence before it, its warp) wrote to shared memory
-// with ordinary stores.  Costs about a microsecond; used only where such stores happened.
+// The same arrival with release semantics at cluster scope: the waiter in the other CTA (which waits
+// with mbar_wait_cluster) may consume what this thread (and, through the fence before it, its warp)
+// wrote to shared memory with ordinary stores.  Costs about a microsecond; used only where such
+// stores happened, by a warp that nothing else waits for.
 __device__ __forceinline__ void mbar_arrive_remote_release(uint64_t* bar, uint32_t cta) {
   asm volatile(
       "{\n\t.reg .b32 remote;\n\t"
@@ -146,6 +147,35 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   const long long start = clock64();
   for (uint32_t round = 1;; ++round) {
     if (mbar_try(bar, parity)) return true;
+    if ((round & 7u) != 0) continue;
+    if (*abort_flag) return false;
+    if (clock64() - start > B200_WAIT_LIMIT_CYCLES) {
+      *abort_flag = 1;
+      report_error(status, ERR_WAIT_TIMEOUT, where, (int)parity);
+      return false;
+    }
+  }
+}
+
+// The same with acquire semantics at cluster scope: for what a thread of another CTA wrote before its
+// mbar_arrive_remote_release.
+__device__ __forceinline__ bool mbar_try_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  int* status, int where) {
+  if (mbar_try_cluster(bar, parity)) return true;
+  const long long start = clock64();
+  for (uint32_t round = 1;; ++round) {
+    if (mbar_try_cluster(bar, parity)) return true;
     if ((round & 7u) != 0) continue;
     if (*abort_flag) return false;
     if (clock64() - start > B200_WAIT_LIMIT_CYCLES) {

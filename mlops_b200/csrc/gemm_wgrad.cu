@@ -822,7 +822,7 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
   uint64_t* bars = reinterpret_cast<uint64_t*>(store_base + Cfg::kStoreBytes);
   uint64_t* landed = bars;                         // [stages] this CTA's TMA bytes
   uint64_t* ready = bars + kStages;            // [stages] leader only: both CTAs' tiles usable
-  uint64_t* empty = bars + 2 * kStages;        // [stages] stage consumed (leader's commit, both CTAs)
+  uint64_t* empty = bars + 2 * kStages;        // [stages] stage consumed (leader's commit, both CTAs) and seen by warp 2
   uint64_t* tfull = bars + 3 * kStages;        // [2] accumulator complete (leader's commit, both CTAs)
   uint64_t* tempty = bars + 3 * kStages + 2;   // [2] leader only: both CTAs drained the buffer
   uint64_t* drain = bars + 3 * kStages + 4;
@@ -845,7 +845,7 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&landed[s], 1);
       mbar_init(&ready[s], 2);   // one arrival per CTA of the pair
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], 2);   // the leader's commit and this CTA's warp 2
     }
     mbar_init(&tfull[0], 1);
     mbar_init(&tfull[1], 1);
@@ -933,7 +933,8 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
       }
     }
   } else if (warp == 1) {
-    // ---- every CTA: wait for its tiles, zero the K tail, report to the leader.
+    // ---- every CTA: wait for its tiles and report them to the leader, except blocks with a K tail.
+    // (A stage that was only written by TMA needs no release from this thread.)
     uint32_t it = 0;
     bool ok = true;
     for (long long t = pair; t < total_tiles && ok; t += num_pairs) {
@@ -946,9 +947,37 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait_warp(&landed[s], ph, abort_flag, p.status, 32)) { ok = false; break; }
+          if (lane == 0 && hi - lo - kb * kWgBlockK >= kWgBlockK) mbar_arrive_remote(&ready[s], 0);
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ---- every CTA: zero the K tail of both operands (see the single-CTA kernel: this CTA's two G and
+    // two X panels) and report the block.  The proxy fence makes the zeros visible to the async proxy;
+    // that the leader's multiplication, which also reads the other CTA's tiles, comes after them takes a
+    // release and an acquire at cluster scope.  The release lasts a microsecond or more, and nearly every
+    // tile of a ragged table ends in a tail: in warp 1 it held back the reports of the blocks behind it.
+    // This warp follows every block and has a say in when its stage is free, so that it is never a round
+    // of stages behind and the parity it waits for is unambiguous.  Rows drawn evenly over the groups, us,
+    // release in warp 1 / here:
+    //   128 groups, 32768 rows, 1536 x 2048   fp32 395 / 381    bf16 326 / 312
+    //    64 groups, 65536 rows, 4096 x 7168   fp32 3890 / 3760  bf16 3160 / 3160
+    // (Handing tails from warp 1 to this one took 375, 283, 3805 and 3295; loading a tail's rows in boxes of
+    // 16, 4 and 1 rows and zeros from a page, with no ordinary stores at all, 353, 342, 3800 and 3430.)
+    uint32_t it = 0;
+    bool ok = true;
+    for (long long t = pair; t < total_tiles && ok; t += num_pairs) {
+      const int g = (int)(t / tiles_per_group);
+      for (int seg = 0; seg < p.segments && ok; ++seg) {
+        int lo, hi;
+        group_range(g, seg, lo, hi);
+        const int num_kb = (hi - lo + kWgBlockK - 1) / kWgBlockK;
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const int s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1;
+          if (!mbar_wait_warp(&landed[s], ph, abort_flag, p.status, 36)) { ok = false; break; }
           const int valid = hi - lo - kb * kWgBlockK;
           if (valid < kWgBlockK) {
-            // both operands (see the single-CTA kernel): this CTA's two G and two X panels
             const int nbytes = (kWgBlockK - valid) * 128;
             for (int pnl = 0; pnl < 4; ++pnl) {
               uint8_t* base = (pnl < 2 ? sA + s * kPairABytes + pnl * kWgPanelBytes
@@ -957,23 +986,13 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
                 *reinterpret_cast<uint4*>(base + o) = make_uint4(0, 0, 0, 0);
             }
             fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (leader) mbar_arrive(&ready[s]);
+              else mbar_arrive_remote_release(&ready[s], 0);
+            }
           }
-          __syncwarp();
-          // A stage that was only written by TMA needs no release from this thread.  One whose
-          // tail rows this warp zeroed was made visible to the async proxy by the fence above;
-          // the PTX memory model would additionally want a cluster-scope release here before the
-          // leader's MMA may depend on those stores.  That arrival costs about a microsecond and
-          // was measured at 19% of this kernel's time (one tail block per tile), so it is a
-          // build option (-DB200_WGRAD_RELEASE_TAIL_ARRIVE); the default relies on the remote
-          // arrival being delivered after this warp's earlier shared-memory stores, which holds
-          // on sm_100 hardware (the results are bit-identical) but is not promised by the model.
-          if (lane == 0) {
-#ifdef B200_WGRAD_RELEASE_TAIL_ARRIVE
-            if (valid < kWgBlockK) mbar_arrive_remote_release(&ready[s], 0);
-            else
-#endif
-              mbar_arrive_remote(&ready[s], 0);
-          }
+          if (lane == 0) mbar_arrive(&empty[s]);
         }
       }
     }
@@ -999,7 +1018,8 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
         for (int done_kb = 0; done_kb < total_kb; ++done_kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
-          if (!mbar_wait(&ready[s], ph, abort_flag, p.status, 34)) { ok = false; break; }
+          // (acquires at cluster scope: a K tail was zeroed by a thread of either CTA)
+          if (!mbar_wait_cluster(&ready[s], ph, abort_flag, p.status, 34)) { ok = false; break; }
           tc_fence_after_sync();
           const uint64_t adesc = make_smem_desc(smem_u32(sA + s * kPairABytes), kWgPanelBytes, 1024);
           const uint64_t bdesc = make_smem_desc(smem_u32(sB + s * kPairBBytes), kWgPanelBytes, 1024);

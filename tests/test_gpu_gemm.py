@@ -259,6 +259,40 @@ def test_wgrad_groups_are_isolated_from_a_neighbours_inf_and_nan(m, n):
     assert torch.equal(dirty[2][:, keep.to(DEV)], clean[2][:, keep.to(DEV)])
 
 
+@pytest.mark.parametrize("segments", [1, 3])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_wgrad_of_many_ragged_groups_beside_poisoned_ones(out_dtype, segments):
+    """Every other group is all Inf and NaN, and nearly every group ends inside a K block (one block and
+    less up to more blocks than there are stages): the clean groups are the bytes of a run without the
+    poison, time after time, and right against float64."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(segments)
+    groups, m, n = 60, 520, 264
+    counts = torch.randint(0, 90, (segments * groups,), generator=g)
+    counts[4], counts[10], counts[11] = 700, 64, 1
+    offsets = torch.zeros(segments * groups + 1, dtype=torch.int32)
+    offsets[1:] = counts.cumsum(0).to(torch.int32)
+    rows = int(offsets[-1])
+    left, right = torch.randn(rows, m, generator=g).bfloat16(), torch.randn(rows, n, generator=g).bfloat16()
+    group_of = torch.repeat_interleave(torch.arange(segments * groups) % groups, counts)
+    bad_left, bad_right = left.clone(), right.clone()
+    bad_left[group_of % 2 == 1], bad_right[group_of % 2 == 1] = float("nan"), float("inf")
+    run = lambda a, b: ops.grouped_wgrad(a.to(DEV), b.to(DEV), offsets.to(DEV), groups, out_dtype)  # noqa: E731
+    clean = run(left, right)
+    for group in range(0, groups, 6):
+        mine = group_of == group
+        expected = left[mine].double().t() @ right[mine].double()
+        magnitude = left[mine].double().abs().t() @ right[mine].double().abs()
+        # exact products; each of `count` additions (and the alignment of the 16 of a multiplication) may
+        # drop 2^-23 of a partial sum, which the sum of magnitudes bounds; then one rounding to bf16 (2^-8)
+        slack = (int(mine.sum()) + 16) * 2.0 ** -23 * magnitude
+        bound = 2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0
+        assert ((clean[group].cpu().double() - expected).abs() <= bound * expected.abs() + slack).all()
+    for _ in range(10):
+        assert torch.equal(run(bad_left, bad_right)[0::2], clean[0::2])
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("b_mn_major", [False, True])
 @pytest.mark.parametrize(
     "counts,n,k",

@@ -2,6 +2,8 @@
 (the kernels are compared with it on the GPU in test_gpu_routing.py), argument validation, the
 expert-parallel index arithmetic."""
 
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -108,3 +110,19 @@ def test_deduplicated_dispatch_reproduces_the_row_per_assignment_layout(world, l
         segment_rows = [sum(1 for row in expected if row[0] == s and row[1] == e)
                         for s in range(world) for e in range(local)]
         assert (offsets[1:] - offsets[:-1]).tolist() == segment_rows
+
+
+def test_ordinary_stores_cross_the_cta_pair_by_release_and_acquire_at_cluster_scope():
+    """The pair kernel of the weight gradient zeroes K tails with ordinary stores that the other CTA's
+    multiplication reads. Whether an arrival of CTA scope would do cannot be seen from results, so the
+    source is held to the rule: the report that follows the zeros is a release at cluster scope (a local
+    arrival in the leader itself), under no build option, and the issuer acquires at cluster scope."""
+    source = (Path(layer.__file__).parent / "csrc" / "gemm_wgrad.cu").read_text()
+    kernel = source[source.index("grouped_wgrad_pair_kernel(const"):source.index("static int launch_pair")]
+    assert "#if" not in kernel[:kernel.index("} else if (warp >= 4)")]
+    zeros = kernel.index("make_uint4(0, 0, 0, 0)")
+    issuer = kernel.index("} else if (warp == 3)")
+    report = kernel[zeros:issuer]
+    assert "if (leader) mbar_arrive(&ready[s]);\n" in report
+    assert "else mbar_arrive_remote_release(&ready[s], 0);" in report and "mbar_arrive_remote(" not in report
+    assert "mbar_wait_cluster(&ready[s]" in kernel[issuer:] and "mbar_wait(&ready[s]" not in kernel[issuer:]
