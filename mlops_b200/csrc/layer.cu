@@ -13,13 +13,14 @@
 
 namespace b200 {
 
-// The frequencies the auxiliary loss's gradient needs, from the sort's offsets.
-__global__ void frequency_kernel(const int* __restrict__ offsets, int experts, float assignments, int sigmoid,
+// The frequencies the auxiliary loss's gradient needs, from the sort's offsets (bit for bit what torch
+// gives for the quotients: it multiplies by the rounded reciprocal of the number of assignments).
+__global__ void frequency_kernel(const int* __restrict__ offsets, int experts, float per_assignment, int sigmoid,
                                  float* __restrict__ frequency) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= experts) return;
   const float count = (float)(offsets[e + 1] - offsets[e]);
-  frequency[e] = sigmoid ? __fdiv_rn(count * (float)experts, assignments) : __fdiv_rn(count, assignments);
+  frequency[e] = (sigmoid ? count * (float)experts : count) * per_assignment;
 }
 
 // Pieces of a workspace, each on a 256-byte boundary.
@@ -146,11 +147,11 @@ extern "C" int b200moe_backward_fp8(const b200moe_backward_args* a, void* stream
   B200_STEP(b200moe_combine(a->rows, D, R, a->slots, nullptr, nullptr, 0, a->grad_x, D, T, D, K, stream));
   const bool sigmoid = a->mode == B200MOE_ROUTE_SIGMOID_NOAUX_TC;
   if (a->grad_aux != nullptr) {
-    frequency_kernel<<<(E + 255) / 256, 256, 0, cuda_stream>>>(a->offsets, E, (float)R, sigmoid, s.frequency);
+    frequency_kernel<<<(E + 255) / 256, 256, 0, cuda_stream>>>(a->offsets, E, 1.0f / (float)R, sigmoid, s.frequency);
     B200_STEP(launch_status());
   }
   return launch_routing_gradient(a->logits, E, T, E, K, a->mode, a->ids, a->route_weights, s.grad_route_weights,
                                  a->grad_aux, a->grad_aux != nullptr ? s.frequency : nullptr,
-                                 sigmoid ? 1.0f / (float)T : (float)E / (float)T, a->grad_probability_sum,
+                                 (float)((sigmoid ? 1.0 : (double)E) / (double)T), a->grad_probability_sum,
                                  a->grad_logits, E, a->grad_logits_high, a->grad_logits_low, cuda_stream);
 }

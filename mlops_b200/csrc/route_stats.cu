@@ -95,9 +95,11 @@ probability_partials_kernel(const float* __restrict__ logits, long long ld, long
 // One block, a thread per expert.  With `counts` also the auxiliary loss of one sequence:
 //   softmax modes  experts * sum_e (counts_e / assignments) * (psum_e / tokens)
 //   sigmoid mode   sum_e (counts_e * experts / assignments) * (psum_e / tokens)
+// The quotients are products with the rounded reciprocals, as torch divides a tensor by a number: the
+// frequencies are those of the step-by-step form to the bit; the sum over the experts has its own order.
 __global__ void __launch_bounds__(1024)
 probability_finish_kernel(const float* __restrict__ partials, int blocks, int E, float* __restrict__ psum,
-                          const long long* __restrict__ counts, float assignments, float tokens, int sigmoid,
+                          const long long* __restrict__ counts, float per_assignment, float per_token, int sigmoid,
                           float* __restrict__ aux) {
   __shared__ float sums[32];
   const int e = threadIdx.x;
@@ -110,8 +112,7 @@ probability_finish_kernel(const float* __restrict__ partials, int blocks, int E,
   if (counts == nullptr) return;
   if (e < E) {
     const float count = (float)counts[e];
-    const float frequency = sigmoid ? __fdiv_rn(count * (float)E, assignments) : __fdiv_rn(count, assignments);
-    v = frequency * __fdiv_rn(v, tokens);
+    v = (sigmoid ? count * (float)E : count) * per_assignment * (v * per_token);
   }
   v = warp_sum(v);
   if ((e & 31) == 0) sums[e >> 5] = v;
@@ -276,7 +277,8 @@ int b200::launch_routing_statistics(const float* logits, long long ld, long long
   B200_DISPATCH_EPL(experts, CALL_PARTIALS);
 #undef CALL_PARTIALS
   probability_finish_kernel<<<1, (experts + 31) / 32 * 32, 0, s>>>(partials, (int)blocks, experts, probability_sum,
-                                                                   counts, (float)(tokens * top_k), (float)tokens,
+                                                                   counts, 1.0f / (float)(tokens * top_k),
+                                                                   1.0f / (float)tokens,
                                                                    mode == 2, aux);
   return launch_status();
 }

@@ -354,11 +354,9 @@ def test_layer_on_a_device_that_is_not_current():
 def test_the_one_call_layer_equals_the_step_by_step_form(monkeypatch, tokens, width, inner, experts, top_k, mode,
                                                          limit, wdtype):
     """`forward_fp8` / `backward_fp8` against the same layer with every launch timed (which takes the
-    steps one by one): the same bytes, but for the auxiliary loss, an [experts]-sized fp32 sum formed
-    in another order (at most `experts` roundings of 2^-24 apart), and what follows from its
-    cotangent: the experts' frequencies are divided here and multiplied by a reciprocal there, a
-    rounding of 2^-24 that may turn single bf16 roundings of the input gradient (2^-8 of a value, few
-    of them: 2^-10 in the 2-norm) and passes into the router's gradient in two bf16 pieces (2^-14)."""
+    steps one by one): the same bytes, gradients of the auxiliary loss included, but for the loss
+    itself, an [experts]-sized fp32 sum formed in another order (at most `experts` roundings of 2^-24
+    apart)."""
     from mlops_b200 import layer, ops
 
     g = torch.Generator(device=DEV).manual_seed(tokens)
@@ -382,9 +380,6 @@ def test_the_one_call_layer_equals_the_step_by_step_form(monkeypatch, tokens, wi
             patch.setattr(ops, "GEMM_TIMINGS", [])
             steps, step_grads = both_passes(**needs)
         torch.testing.assert_close(res[1], steps[1], rtol=experts * 2.0 ** -23, atol=0)
-        for one, other in zip((res[0], *res[2:], *grads[0], *grads[1]), (steps[0], *steps[2:], *step_grads[0], *step_grads[1])):
+        for one, other in zip((res[0], *res[2:], *sum(grads, ())), (steps[0], *steps[2:], *sum(step_grads, ()))):
             assert one.dtype == other.dtype and torch.equal(one, other)
-        for one, other in zip(grads[2], step_grads[2]):
-            bound = 2.0 ** -14 if one.dtype == torch.float32 else 2.0 ** -10
-            assert (one.float() - other.float()).norm() <= bound * other.float().norm()
     ops.check_status(DEV)
