@@ -465,8 +465,9 @@ __device__ __forceinline__ Float2 mad2(Float2 a, Float2 b, Float2 c) {
   return r;
 }
 
-// E4M3 bytes of clamp(v / scale, +-448) with the division rounded to nearest, i.e. exactly
-// what `x / scale` followed by the cast gives on a CPU.  Fast path: multiply by the rounded
+// E4M3 bytes of v / scale with the division rounded to nearest and the cast saturating at +-448, i.e.
+// exactly what `x / scale`, clamped, followed by the cast gives on a CPU; a NaN stays a NaN whatever its
+// neighbours are (no explicit clamp: fminf and fmaxf would make it +-448).  Fast path: multiply by the rounded
 // reciprocal; the true quotient lies within 2^-22 (relative) of that product, and the cast is
 // monotonic, so when both ends of the interval [q(1-2^-21), q(1+2^-21)] cast to the same
 // byte that byte is the exact answer.  Otherwise (a value within an ulp of an E4M3 rounding
@@ -491,9 +492,7 @@ __device__ __forceinline__ uint2 quantize8(const float (&v)[8], float scale) {
     w[0] = w[1] = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      float q = __fdiv_rn(v[i], scale);
-      q = fminf(fmaxf(q, -448.0f), 448.0f);
-      w[i >> 2] |= (uint32_t)to_e4m3(q) << (8 * (i & 3));
+      w[i >> 2] |= (uint32_t)to_e4m3(__fdiv_rn(v[i], scale)) << (8 * (i & 3));
     }
   }
   return make_uint2(w[0], w[1]);

@@ -420,8 +420,7 @@ quantize_blocks_kernel(const SrcT* __restrict__ w, int out, int in, int blocks_o
     if (!exact) {
 #pragma unroll
       for (int k = 0; k < kVec; ++k) {
-        const float v = fminf(fmaxf(__fdiv_rn(value(i, k), s), -448.0f), 448.0f);
-        const uint32_t byte = (uint32_t)to_e4m3(v) << (8 * (k & 3));
+        const uint32_t byte = (uint32_t)to_e4m3(__fdiv_rn(value(i, k), s)) << (8 * (k & 3));
         packed[k >> 2] = (k & 3) ? packed[k >> 2] | byte : byte;
       }
     }
@@ -470,9 +469,7 @@ quantize_blocks_general_kernel(const SrcT* __restrict__ w, int out, int in, int 
     for (int k = 0; k < 4; ++k) {
       const int col = bc * 128 + tc * 4 + k;
       if (col < in) {
-        float v = __fdiv_rn((float)base[(long long)row * in + col], s);
-        v = fminf(fmaxf(v, -448.0f), 448.0f);
-        qbase[(long long)row * in + col] = to_e4m3(v);
+        qbase[(long long)row * in + col] = to_e4m3(__fdiv_rn((float)base[(long long)row * in + col], s));
       }
     }
   }
@@ -586,9 +583,7 @@ column_cast_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int rows,
       w[0] = w[1] = 0;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        float qv = __fdiv_rn(v[i], sc[i]);
-        qv = fminf(fmaxf(qv, -448.0f), 448.0f);
-        w[i >> 2] |= (uint32_t)to_e4m3(qv) << (8 * (i & 3));
+        w[i >> 2] |= (uint32_t)to_e4m3(__fdiv_rn(v[i], sc[i])) << (8 * (i & 3));
       }
     }
     *reinterpret_cast<uint2*>(q + (long long)r * ldq + c) = make_uint2(w[0], w[1]);

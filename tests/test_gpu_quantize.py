@@ -35,7 +35,7 @@ def test_weight_blocks_of_aligned_and_unaligned_sources(shape, dtype, special):
     """The one-pass quantiser (16-byte loads) writes the bytes and scales of the value-by-value one,
     which serves a source one element off alignment; both equal the oracle where it is defined by
     finite values. Infinities and NaN: the maximum skips a NaN, an infinity makes the scale
-    infinite, and a NaN quotient is stored as -448."""
+    infinite, and a NaN quotient stays a NaN."""
     ops = _ops()
     g = torch.Generator().manual_seed(sum(shape))
     n = shape[0] * shape[1] * shape[2]
@@ -241,6 +241,35 @@ def test_swiglu_over_the_whole_range_of_gates(rows, width, limit):
     assert (error <= expected.abs()[~odd] * (2.0 ** -8 + 2.0 ** -20) + 1e-37).all()
     if limit is None:
         assert actual[0, 2].isnan() and actual[0, 0].isinf() and actual[0, 1].isnan()
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("boundary", [True, False])
+def test_a_nan_survives_every_quantiser_whatever_its_neighbours(value, boundary):
+    """A NaN, or an infinity divided by its infinite scale, among eight values of which one lies on a
+    rounding boundary of E4M3 (17 between 16 and 18 at scale 1: these eight are divided exactly) or none
+    does: the NaN byte, and the other values as torch's division, clamp and cast give them at the
+    kernel's scale."""
+    ops = _ops()
+    x = torch.randn(128, 128, generator=torch.Generator().manual_seed(3)).bfloat16()
+    x[:, 0], x[:, 1], x[:, 2] = 448.0, 17.0 if boundary else 16.0, value  # scale 1 unless infinite
+    wide = x.to(DEV)
+    slots = torch.arange(128, dtype=torch.int32, device=DEV).view(128, 1)
+    whole = torch.tensor([0, 128], dtype=torch.int32, device=DEV)
+    store = torch.empty(128 * 128 + 1, dtype=torch.bfloat16, device=DEV)
+    store[1:] = wide.view(-1)
+    produced = {
+        "1x128": ops.quantize_rows(wide), "row": ops.quantize_rows(wide, mode="row"),
+        "scatter": ops.quantize_rows_scatter(wide, slots), "columns": ops.quantize_columns(wide, whole, 1),
+        "blocks": [t[0] for t in ops.quantize_blocks(wide[None])],
+        "blocks fp32": [t[0] for t in ops.quantize_blocks(wide.float()[None])],
+        "blocks, unaligned": [t[0] for t in ops.quantize_blocks(store[1:].view(1, 128, 128))],
+    }
+    for name, (q, scale) in produced.items():
+        got = q.cpu().float()
+        expected = torch.clamp(x.float() / scale.cpu().float(), -448.0, 448.0).to(torch.float8_e4m3fn).float()
+        assert expected[:, 2].isnan().all() and torch.equal(got.isnan(), expected.isnan()), name
+        assert torch.equal(got.nan_to_num(0.0), expected.nan_to_num(0.0)), name
 
 
 @pytest.mark.parametrize("limit", [None, 1.3])
