@@ -450,7 +450,8 @@ int b200moe_gather_scalar(const float* values, long long n_values, const int32_t
  * The block-FP8 layer in one call per direction: the kernels of the entry points above, in the
  * order a caller would enqueue them.  width and inner are multiples of 128, experts <= 1024,
  * 0 < top_k <= min(experts, 32), tokens > 0; R = tokens * top_k rows.  Every matrix is dense, every
- * pointer as aligned as the single entry points want it.
+ * pointer as aligned as the single entry points want it.  A missing or misaligned pointer, a bad size or
+ * a bad mode is refused before the first launch.
  *
  * Forward, after the router GEMM (logits fp32 [tokens, experts]): route, sort, quantise, up GEMM,
  * SwiGLU, down GEMM, combine, statistics of one sequence (aux, probability_sum).

@@ -7,6 +7,8 @@
 //
 // No step reads device memory on the host or allocates: the caller hands over every result and
 // scratch buffer (sizes beside the declarations in include/b200moe.h).
+#include <initializer_list>
+
 #include "common.cuh"
 #include "host_util.h"
 #include "../../include/b200moe.h"
@@ -70,6 +72,22 @@ static bool sizes_ok(long long tokens, int width, int inner, int experts, int to
          experts <= 1024 && top_k > 0 && top_k <= 32 && top_k <= experts && tokens * top_k <= 0x7fffffffLL;
 }
 
+static bool mode_ok(int mode) { return mode >= B200MOE_ROUTE_TOPK_THEN_SOFTMAX && mode <= B200MOE_ROUTE_SIGMOID_NOAUX_TC; }
+
+// The pointers of a call are looked at before its first launch: a missing or misaligned one must not
+// show up when part of the work is on the stream already.
+static bool all_given(std::initializer_list<const void*> pointers) {
+  for (const void* p : pointers)
+    if (p == nullptr) return false;
+  return true;
+}
+
+static bool all_aligned(uintptr_t bytes, std::initializer_list<const void*> pointers) {  // (NULL is aligned)
+  for (const void* p : pointers)
+    if ((uintptr_t)p % bytes) return false;
+  return true;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -86,8 +104,15 @@ extern "C" long long b200moe_forward_workspace_bytes(long long tokens, int width
 }
 
 extern "C" int b200moe_forward_fp8(const b200moe_forward_args* a, void* stream) {
-  if (a == nullptr || !a->workspace || !a->aux || !a->counts) return B200MOE_ERR_ARG;
-  if (!sizes_ok(a->tokens, a->width, a->inner, a->experts, a->top_k)) return B200MOE_ERR_ARG;
+  if (a == nullptr || !sizes_ok(a->tokens, a->width, a->inner, a->experts, a->top_k) || !mode_ok(a->mode))
+    return B200MOE_ERR_ARG;
+  if (!all_given({a->x, a->residual, a->logits, a->w13, a->w13_scale, a->w2, a->w2_scale, a->route_weights, a->ids,
+                  a->order, a->offsets, a->slots, a->counts, a->h13, a->output, a->aux, a->probability_sum, a->x_q,
+                  a->act_q, a->expert_rows, a->workspace, a->status}))
+    return B200MOE_ERR_ARG;
+  if (!all_aligned(16, {a->x, a->residual, a->w13, a->w2, a->h13, a->output, a->x_q, a->act_q, a->expert_rows}) ||
+      !all_aligned(256, {a->workspace}))
+    return B200MOE_ERR_ALIGN;
   const int D = a->width, F = a->inner, E = a->experts, K = a->top_k;
   const long long T = a->tokens, R = T * K;
   const ForwardScratch s((char*)a->workspace, T, D, F, E, K);
@@ -116,9 +141,17 @@ extern "C" long long b200moe_backward_workspace_bytes(long long tokens, int widt
 }
 
 extern "C" int b200moe_backward_fp8(const b200moe_backward_args* a, void* stream) {
-  if (a == nullptr || !a->workspace || !a->rows || !a->r) return B200MOE_ERR_ARG;
-  if (!sizes_ok(a->tokens, a->width, a->inner, a->experts, a->top_k)) return B200MOE_ERR_ARG;
-  if (a->grad_w13 != nullptr && a->gh == nullptr) return B200MOE_ERR_ARG;
+  if (a == nullptr || !sizes_ok(a->tokens, a->width, a->inner, a->experts, a->top_k) || !mode_ok(a->mode))
+    return B200MOE_ERR_ARG;
+  if (!all_given({a->grad_output, a->x, a->w13, a->w13_scale, a->w2, a->w2_scale, a->logits, a->route_weights, a->ids,
+                  a->order, a->offsets, a->slots, a->h13, a->grad_x, a->grad_logits, a->grad_logits_high,
+                  a->grad_logits_low, a->dy_q, a->rows, a->r, a->gh_q, a->workspace, a->status}) ||
+      (a->grad_w13 != nullptr && a->gh == nullptr))
+    return B200MOE_ERR_ARG;
+  if (!all_aligned(16, {a->grad_output, a->x, a->w13, a->w2, a->h13, a->grad_x, a->grad_w13, a->grad_w2, a->dy_q,
+                        a->rows, a->r, a->gh_q, a->gh}) ||
+      !all_aligned(256, {a->workspace}))
+    return B200MOE_ERR_ALIGN;
   const int D = a->width, F = a->inner, E = a->experts, K = a->top_k;
   const long long T = a->tokens, R = T * K;
   const BackwardScratch s((char*)a->workspace, T, D, F, E, K);

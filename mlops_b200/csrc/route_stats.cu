@@ -268,6 +268,7 @@ extern "C" int b200moe_routing_probability_sum(const float* logits, long long ld
 int b200::launch_routing_statistics(const float* logits, long long ld, long long tokens, int experts, int mode,
                                     void* workspace, float* probability_sum, const long long* counts, int top_k,
                                     float* aux, cudaStream_t s) {
+  if (!logits || !workspace || !probability_sum || (counts != nullptr && aux == nullptr)) return B200MOE_ERR_ARG;
   const long long blocks = stat_blocks(tokens);
   const long long per_block = (tokens + blocks - 1) / blocks;
   float* partials = reinterpret_cast<float*>(workspace);

@@ -67,6 +67,32 @@ def test_argument_validation_needs_no_gpu():
     assert lib.b200moe_combine(None, 0, 0, None, None, None, 0, None, 0, 0, 8, 1, None) == -1
 
 
+def test_the_layer_calls_refuse_every_missing_pointer_before_any_launch():
+    """Each required pointer of the two layer calls cleared in turn, a mode out of range, a misaligned
+    pointer: an error before the first launch, so the (invented) addresses are never used. Optional
+    pointers are those the header lets a caller leave out."""
+    from mlops_b200._lib import BackwardArgs, ForwardArgs, lib
+
+    sizes = dict(tokens=4, width=256, inner=128, experts=8, top_k=2)
+    for struct, call, optional in (
+            (ForwardArgs, lib.b200moe_forward_fp8, {"bias"}),
+            (BackwardArgs, lib.b200moe_backward_fp8,
+             {"grad_aux", "grad_probability_sum", "grad_w13", "grad_w2"})):
+        pointers = [name for name, kind in struct._fields_ if kind is ctypes.c_void_p]
+
+        def filled(**changes):
+            fields = {**sizes, "mode": 1, **{name: 4096 for name in pointers}, **changes}
+            return ctypes.byref(struct(**fields))
+
+        for name in pointers:
+            if name not in optional:
+                assert call(filled(**{name: None}), None) == -1, name
+        assert call(filled(mode=3), None) == -1 and call(filled(mode=-1), None) == -1
+        assert call(filled(tokens=0), None) == -1 and call(filled(inner=100), None) == -1
+        for name in ("x", "h13", "workspace"):
+            assert call(filled(**{name: 4096 + 8}), None) == -2, name
+
+
 def test_ops_refuse_cpu_tensors():
     import pytest
     import torch
