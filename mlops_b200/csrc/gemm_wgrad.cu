@@ -808,7 +808,7 @@ struct PairCfg {
 };
 constexpr int kPairBlockM = 256;  // per pair
 
-template <typename OutT>
+template <typename OutT, bool ACCUMULATE>
 __global__ void __launch_bounds__(kWgThreads, 1)
 grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __grid_constant__ CUtensorMap tmap_x,
                           const WgradParams p) {
@@ -1087,7 +1087,11 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
         const int cols = min(32, p.N - (col0 + cc * 32));  // of this chunk inside the matrix (a multiple of 8)
-        if (p.accumulate) {
+        // Adding to a caller's buffer is an instantiation of its own: with both stores in one kernel the
+        // plain one was up to 10% slower (128 groups of 256 rows, 1536 x 2048, bf16: 261 / 236 us).  It stores a
+        // row per lane and does not use the buffer below; six operand stages in the buffer's place gave
+        // nothing (the same shape fp32: 1022 us with five and with six).
+        if constexpr (ACCUMULATE) {
           if (m < p.M && cols > 0) {
             float v[32];
 #pragma unroll
@@ -1143,9 +1147,9 @@ grouped_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmap_g, const __gr
   }
 }
 
-template <typename OutT>
+template <typename OutT, bool ACCUMULATE>
 static int launch_pair(const CUtensorMap& tg, const CUtensorMap& tx, const WgradParams& p, cudaStream_t s) {
-  auto kern = grouped_wgrad_pair_kernel<OutT>;
+  auto kern = grouped_wgrad_pair_kernel<OutT, ACCUMULATE>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<OutT>::kSmemBytes) != cudaSuccess)
     return B200MOE_ERR_LAUNCH;
   const long long tiles = (long long)p.groups * ((p.M + kPairBlockM - 1) / kPairBlockM) *
@@ -1252,7 +1256,9 @@ static int grouped_wgrad_impl(const void* g, long long ldg, const void* x, long 
     return v != nullptr && v[0] == '1';
   }();
   if (!force_single && M > 128 && N > 128) {
-    return out_is_fp32 ? launch_pair<float>(tg, tx, p, s) : launch_pair<__nv_bfloat16>(tg, tx, p, s);
+    if (accumulate)
+      return out_is_fp32 ? launch_pair<float, true>(tg, tx, p, s) : launch_pair<__nv_bfloat16, true>(tg, tx, p, s);
+    return out_is_fp32 ? launch_pair<float, false>(tg, tx, p, s) : launch_pair<__nv_bfloat16, false>(tg, tx, p, s);
   }
   if (!force_single && (M <= kNarrowMax || N <= kNarrowMax))
     return out_is_fp32 ? launch_narrow<float>(tg, tx, p, s) : launch_narrow<__nv_bfloat16>(tg, tx, p, s);

@@ -259,6 +259,30 @@ def test_wgrad_groups_are_isolated_from_a_neighbours_inf_and_nan(m, n):
     assert torch.equal(dirty[2][:, keep.to(DEV)], clean[2][:, keep.to(DEV)])
 
 
+@pytest.mark.parametrize("m,n", [(256, 264), (520, 136), (128, 256)])  # the CTA-pair kernel twice, the single-CTA kernel
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_wgrad_added_to_a_callers_buffer(m, n, out_dtype):
+    """A scaled product added to what a buffer holds, empty and ragged groups included: the float64 sum
+    to one fp32 multiply-add and one rounding."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(m)
+    counts = [0, 70, 1300, 15, 0, 64, 1]
+    rows, groups = sum(counts), len(counts)
+    left, right = torch.randn(rows, m, generator=g).bfloat16(), torch.randn(rows, n, generator=g).bfloat16()
+    start = torch.randn(groups, m, n, generator=g).to(out_dtype)
+    buffer = start.to(DEV)
+    offsets = _offsets(counts)
+    ops.grouped_wgrad(left.to(DEV), right.to(DEV), offsets.to(DEV), groups, accumulate_into=buffer, scale=0.5)
+    ops.check_status(DEV)
+    for group, (lo, hi) in enumerate(zip(offsets[:-1].tolist(), offsets[1:].tolist())):
+        a, b = left[lo:hi].double(), right[lo:hi].double()
+        expected = start[group].double() + 0.5 * (a.t() @ b)
+        # the product as in the test below; one multiply-add (2^-24) and, to bf16, one rounding (2^-8)
+        slack = 0.5 * (counts[group] + 16) * 2.0 ** -23 * (a.abs().t() @ b.abs())
+        bound = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -23
+        assert ((buffer[group].cpu().double() - expected).abs() <= bound * expected.abs() + slack).all()
+
+
 @pytest.mark.parametrize("segments", [1, 3])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_wgrad_of_many_ragged_groups_beside_poisoned_ones(out_dtype, segments):
