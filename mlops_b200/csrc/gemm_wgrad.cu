@@ -44,7 +44,7 @@ struct WgradParams {
   // X ([groups, N]); the product of a group is multiplied by g_scale[m] * x_scale[n] at the store.
   const float* g_scale;
   const float* x_scale;
-  int band;        // pair kernel: M tiles of a group walked together before the next column of tiles (banded_tile)
+  int band = 1;    // pair kernel: M tiles of a group walked together before the next column of tiles (banded_tile)
   int wide_store;  // the output's base and row pitch are multiples of 32 bytes: 32-byte stores
 };
 
@@ -102,14 +102,8 @@ __device__ __forceinline__ void load8<float>(const float* src, float (&v)[8]) {
 
 // The store of eight sums: scaled, and added to what the destination holds when the caller
 // accumulates gradients over several calls (micro-batches) in one buffer.
-// -DB200_WGRAD_ABLATE_STORE=1 (timing experiments only) drops the store: what the epilogue's
-// writes cost the main loop shows as the difference.  The shipped library stores.
-#ifndef B200_WGRAD_ABLATE_STORE
-#define B200_WGRAD_ABLATE_STORE 0
-#endif
 template <typename OutT>
 __device__ __forceinline__ void finish8(OutT* dst, float (&v)[8], float scale, int accumulate) {
-  if (B200_WGRAD_ABLATE_STORE && v[0] != 12345.678f) return;
   if (accumulate) {
     float old[8];
     load8<OutT>(dst, old);
@@ -1328,7 +1322,6 @@ extern "C" int b200moe_grouped_wgrad_fp8(const void* g, long long ldg, const flo
   p.rows_total = (int)rows_total;
   p.segments = segments;
   p.status = status;
-  p.band = tile_band(2 * rows_total / groups * N);
   p.scale = scale;
   p.accumulate = accumulate;
   p.g_scale = g_scale;
