@@ -383,3 +383,45 @@ def test_the_one_call_layer_equals_the_step_by_step_form(monkeypatch, tokens, wi
         for one, other in zip((res[0], *res[2:], *sum(grads, ())), (steps[0], *steps[2:], *sum(step_grads, ()))):
             assert one.dtype == other.dtype and torch.equal(one, other)
     ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("mode,lengths,forward_whole,backward_whole", [
+    ("sigmoid_noaux_tc", None, True, (True, True)), ("sigmoid_noaux_tc", (100, 150, 50), False, (True, False)),
+    ("softmax_then_topk", (100, 150, 50), True, (True, True))])
+def test_the_choice_between_the_forms_of_the_layer_does_not_show(monkeypatch, mode, lengths, forward_whole,
+                                                                 backward_whole):
+    """Group-limited routing and calls of several sequences, where the sigmoid mode's auxiliary loss is
+    one sum per sequence: which direction goes as one call, and the bytes of the step-by-step form in
+    everything but the loss where that is formed by the one call (at most `experts` roundings)."""
+    from mlops_b200 import layer, ops
+
+    tokens, width, inner, experts, top_k = 300, 256, 128, 64, 6
+    g = torch.Generator(device=DEV).manual_seed(len(mode))
+    randn = lambda *s, std=1.0: torch.randn(*s, generator=g, device=DEV) * std  # noqa: E731
+    x, residual, dy = (randn(tokens, width).bfloat16() for _ in range(3))
+    router, bias = randn(experts, width, std=0.1), randn(experts, std=0.01)
+    w13, w2 = ops.quantize_blocks(randn(experts, 2 * inner, width, std=0.1)), ops.quantize_blocks(
+        randn(experts, width, inner, std=0.1))
+    d_aux, d_psum = randn(()), randn(experts)
+    calls = []
+    for name in ("forward_fp8", "backward_fp8"):
+        one_call = getattr(ops, name)
+        monkeypatch.setattr(ops, name, lambda *a, _name=name, _call=one_call, **k: (calls.append(_name), _call(*a, **k))[1])
+
+    def both_passes():
+        calls.clear()
+        res = layer.forward_routed(x, residual, router, w13, w2, top_k=top_k, routing_mode=mode, router_bias=bias,
+                                   n_group=8, topk_group=3, routed_scaling=2.5, lengths=lengths)
+        grads = [layer.backward_routed(dy, aux, d_psum, x, router, w13, w2, *res[4:], top_k=top_k, routing_mode=mode,
+                                       lengths=lengths) for aux in (None, d_aux)]
+        return res, grads, list(calls)
+
+    res, grads, taken = both_passes()
+    assert taken == ["forward_fp8"] * forward_whole + ["backward_fp8"] * sum(backward_whole)
+    monkeypatch.setattr(ops, "GEMM_TIMINGS", [])
+    steps, step_grads, taken = both_passes()
+    assert taken == []
+    torch.testing.assert_close(res[1], steps[1], rtol=experts * 2.0 ** -23 if forward_whole else 0.0, atol=0)
+    for one, other in zip((res[0], *res[2:], *sum(grads, ())), (steps[0], *steps[2:], *sum(step_grads, ()))):
+        assert one.dtype == other.dtype and torch.equal(one, other)
+    ops.check_status(DEV)
