@@ -361,7 +361,7 @@ extern "C" int b200moe_grouped_gemm_bf16(const void* a, long long lda, const voi
   p.K = K;
   p.rows_total = (int)rows_total;
   p.weights = weights;
-  p.band = tile_band(2LL * N * K);
+  p.band = tile_band(2LL * N * K, rows_total, groups);
   p.alpha = alpha;
   p.status = status;
   // upper bound of the tile count: every group may end in a partial tile

@@ -1344,7 +1344,7 @@ static int grouped_gemm_fp8_impl(const void* a, long long lda, const float* a_sc
   p.K = K;
   p.rows_total = (int)rows_total;
   p.weights = weights;
-  p.band = tile_band((long long)N * K);
+  p.band = tile_band((long long)N * K, rows_total, groups);
   p.act_q = nullptr;
   p.ldq = 0;
   p.act_scale = nullptr;
@@ -1522,7 +1522,7 @@ extern "C" int b200moe_grouped_gemm_fp8_swiglu(const void* a, long long lda, con
   p.K = K;
   p.rows_total = (int)rows_total;
   p.weights = weights;
-  p.band = tile_band((long long)N * K);
+  p.band = tile_band((long long)N * K, rows_total, groups);
   p.act_q = reinterpret_cast<uint8_t*>(act_q);
   p.ldq = ldq;
   p.act_scale = act_scale;

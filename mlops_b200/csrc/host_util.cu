@@ -35,8 +35,16 @@ void set_cta_limit(int n) { g_cta_limit = n > 0 ? n : 0; }
 //                           117 MB 5574 / 4091
 //   bf16 GEMM               34 MB 241 / 235   67 MB 512 / 456   117 MB 1006 / 803   235 MB 2257 / 1608
 //   weight gradient         34 MB 2368 / 2424   67 MB 1711 / 1583   117 MB 3230 / 2757
-// Bands of 8 to 32 are within 3% of one another.
+// (one threshold for the three; the bf16 GEMM would gain 2% from a lower one).  Bands of 8 to 32 are
+// within 3% of one another.
 int tile_band(long long bytes) { return bytes > (40LL << 20) ? 16 : 1; }
+
+// Where the groups have less than a whole tile of rows (decoding), nothing is read twice in either order
+// and a band only spreads the tiles in flight over sixteen groups' weights.  Eight groups, 28672 x 4096,
+// column order / bands, in us, by rows in all:
+//   E4M3    128 163 / 167   512 175 / 178   1024 227 / 211   2048 393 / 342
+//   bf16    128 308 / 315   512 317 / 327   1024 407 / 359   2048 685 / 534
+int tile_band(long long bytes, long long rows, int groups) { return rows >= 128LL * groups ? tile_band(bytes) : 1; }
 
 int sm_count_device() {
   static int cached[64];

@@ -29,6 +29,7 @@ EncodeTiledFn get_encode_tiled();
 // Rows of tiles a GEMM walks together (banded_tile): `bytes` is what one row of tiles reads of the
 // operand that runs along it (a group's whole weight, or its rows of X in a weight gradient).
 int tile_band(long long bytes);
+int tile_band(long long bytes, long long rows, int groups);  // ... of a GEMM over `rows` rows in `groups` groups
 // b200moe_routing_probability_sum and, with counts (the sort's, int64) and aux, the auxiliary loss of
 // the rows as one sequence.
 int launch_routing_statistics(const float* logits, long long ld, long long tokens, int experts, int mode,

@@ -699,10 +699,10 @@ def test_tma_store_and_register_store_write_the_same_bytes():
     assert digests[0] == digests[1]
 
 
-@pytest.mark.parametrize("counts", [[2181, 0, 7], [300, 1900]])
+@pytest.mark.parametrize("counts", [[2181, 0, 7], [300, 1900], [40, 0, 343], [40, 0, 344]])
 def test_banded_tile_order_covers_the_same_tiles(counts):
-    """Wide operands (over 40 MB per group) walk their tiles in bands of 16 rows; narrow slices of
-    the same operands do not. Bands that end early (18 and 19 rows of tiles here) included, the
+    """Wide operands (over 40 MB per group) walk their tiles in bands of 16 rows from 128 rows per group on
+    (384 rows in all here); narrow slices of the same operands do not. Bands that end early (18 and 19 rows of tiles here) included, the
     products are the same bytes."""
     ops = _ops()
     rows, k, n, step = sum(counts), 4096, 10752, 3584
