@@ -2,12 +2,16 @@
 // pass up to the router's own gradient.  Each enqueues the same kernels, through the same entry
 // points, as a caller that makes the calls one by one; what goes is the host work between them.
 // From Python the forward pass took 273 us of host time (eight wrapper calls and five
-// [experts]-sized tensor operations, against 88 us of kernels for one decoded token) and takes 140,
-// the backward pass 366 us and takes 181.
+// [experts]-sized tensor operations, against 88 us of kernels for one decoded token) and takes 130,
+// the backward pass 366 us and takes 172.
 //
 // No step reads device memory on the host or allocates: the caller hands over every result and
 // scratch buffer (sizes beside the declarations in include/b200moe.h).
+#include <cstdlib>
+#include <cstring>
 #include <initializer_list>
+
+#include <nvtx3/nvToolsExt.h>
 
 #include "common.cuh"
 #include "host_util.h"
@@ -88,14 +92,33 @@ static bool all_aligned(uintptr_t bytes, std::initializer_list<const void*> poin
   return true;
 }
 
+// B200MOE_NVTX=1: a range around each step's launches, as the Python wrappers have around theirs.
+struct Range {
+  explicit Range(const char* name) {
+    if (wanted()) nvtxRangePushA(name);
+  }
+  ~Range() {
+    if (wanted()) nvtxRangePop();
+  }
+  static bool wanted() {
+    static const bool on = [] {
+      const char* v = getenv("B200MOE_NVTX");
+      return v != nullptr && strcmp(v, "1") == 0;
+    }();
+    return on;
+  }
+};
+
 }  // namespace b200
 
 using namespace b200;
 
-#define B200_STEP(call)                 \
-  do {                                  \
-    const int code_ = (call);           \
-    if (code_ != B200MOE_OK) return code_; \
+// One step through its entry point, in an NVTX range of the wrapper's name where ranges are wanted.
+#define B200_STEP(name, ...)                         \
+  do {                                               \
+    const Range range_("b200moe." #name);            \
+    const int code_ = b200moe_##name(__VA_ARGS__);   \
+    if (code_ != B200MOE_OK) return code_;           \
   } while (0)
 
 extern "C" long long b200moe_forward_workspace_bytes(long long tokens, int width, int inner, int experts, int top_k) {
@@ -116,21 +139,22 @@ extern "C" int b200moe_forward_fp8(const b200moe_forward_args* a, void* stream) 
   const int D = a->width, F = a->inner, E = a->experts, K = a->top_k;
   const long long T = a->tokens, R = T * K;
   const ForwardScratch s((char*)a->workspace, T, D, F, E, K);
-  B200_STEP(b200moe_route_topk(a->logits, E, (int)T, E, K, a->mode, a->bias, a->n_group, a->topk_group,
-                               a->routed_scaling, a->route_weights, a->ids, stream));
-  B200_STEP(b200moe_sort_assignments(a->ids, R, E, a->order, a->offsets, a->slots, a->counts, s.sort, a->status,
-                                     stream));
+  B200_STEP(route_topk, a->logits, E, (int)T, E, K, a->mode, a->bias, a->n_group, a->topk_group,
+            a->routed_scaling, a->route_weights, a->ids, stream);
+  B200_STEP(sort_assignments, a->ids, R, E, a->order, a->offsets, a->slots, a->counts, s.sort, a->status,
+            stream);
   // scales are stored block-major, [width / 128][rows]
-  B200_STEP(b200moe_quantize_rows_scatter(a->x, D, T, a->slots, K, R, D, a->x_q, D, s.x_scale, 1, R, nullptr, D,
-                                          a->status, stream));
-  B200_STEP(b200moe_grouped_gemm_fp8(a->x_q, D, s.x_scale, 1, R, a->w13, a->w13_scale, a->h13, 2LL * F, nullptr, 0,
-                                     a->offsets, E, E, R, 2 * F, D, 0, 256, a->status, stream));
-  B200_STEP(b200moe_swiglu_quantize(a->h13, 2LL * F, R, F, a->act_q, F, s.act_scale, 1, R, nullptr, F, a->limit,
-                                    a->limited, stream));
-  B200_STEP(b200moe_grouped_gemm_fp8(a->act_q, F, s.act_scale, 1, R, a->w2, a->w2_scale, a->expert_rows, D, nullptr, 0,
-                                     a->offsets, E, E, R, D, F, 0, 256, a->status, stream));
-  B200_STEP(b200moe_combine(a->expert_rows, D, R, a->slots, a->route_weights, a->residual, D, a->output, D, T, D, K,
-                            stream));
+  B200_STEP(quantize_rows_scatter, a->x, D, T, a->slots, K, R, D, a->x_q, D, s.x_scale, 1, R, nullptr, D,
+            a->status, stream);
+  B200_STEP(grouped_gemm_fp8, a->x_q, D, s.x_scale, 1, R, a->w13, a->w13_scale, a->h13, 2LL * F, nullptr, 0,
+            a->offsets, E, E, R, 2 * F, D, 0, 256, a->status, stream);
+  B200_STEP(swiglu_quantize, a->h13, 2LL * F, R, F, a->act_q, F, s.act_scale, 1, R, nullptr, F, a->limit,
+            a->limited, stream);
+  B200_STEP(grouped_gemm_fp8, a->act_q, F, s.act_scale, 1, R, a->w2, a->w2_scale, a->expert_rows, D, nullptr, 0,
+            a->offsets, E, E, R, D, F, 0, 256, a->status, stream);
+  B200_STEP(combine, a->expert_rows, D, R, a->slots, a->route_weights, a->residual, D, a->output, D, T, D, K,
+            stream);
+  const Range range("b200moe.routing_statistics");
   return launch_routing_statistics(a->logits, E, T, E, a->mode, s.statistics, a->probability_sum, a->counts, K, a->aux,
                                    reinterpret_cast<cudaStream_t>(stream));
 }
@@ -159,29 +183,31 @@ extern "C" int b200moe_backward_fp8(const b200moe_backward_args* a, void* stream
   // `rows` holds in turn: dy and x in expert order (operands of the weight gradients), the input
   // gradient's rows.  `r` becomes the down weight's second operand in place.
   void* dy_rows = a->grad_w2 != nullptr ? a->rows : nullptr;
-  B200_STEP(b200moe_quantize_rows_scatter(a->grad_output, D, T, a->slots, K, R, D, a->dy_q, D, s.dy_scale, 1, R,
-                                          dy_rows, D, a->status, stream));
-  B200_STEP(b200moe_grouped_gemm_fp8(a->dy_q, D, s.dy_scale, 1, R, a->w2, a->w2_scale, a->r, F, nullptr, 0, a->offsets,
-                                     E, E, R, F, D, 1, 256, a->status, stream));
-  B200_STEP(b200moe_dswiglu_routed(a->h13, 2LL * F, a->r, F, a->route_weights, R, a->order, R, F, s.dscore, a->gh_q,
-                                   2LL * F, s.gh_scale, 1, R, a->gh, 2LL * F, a->grad_w2 != nullptr ? a->r : nullptr, F,
-                                   a->limit, a->limited, a->status, stream));
-  B200_STEP(b200moe_gather_scalar(s.dscore, R, a->slots, R, s.grad_route_weights, a->status, stream));
+  B200_STEP(quantize_rows_scatter, a->grad_output, D, T, a->slots, K, R, D, a->dy_q, D, s.dy_scale, 1, R,
+            dy_rows, D, a->status, stream);
+  B200_STEP(grouped_gemm_fp8, a->dy_q, D, s.dy_scale, 1, R, a->w2, a->w2_scale, a->r, F, nullptr, 0, a->offsets,
+            E, E, R, F, D, 1, 256, a->status, stream);
+  B200_STEP(dswiglu_routed, a->h13, 2LL * F, a->r, F, a->route_weights, R, a->order, R, F, s.dscore, a->gh_q,
+            2LL * F, s.gh_scale, 1, R, a->gh, 2LL * F, a->grad_w2 != nullptr ? a->r : nullptr, F,
+            a->limit, a->limited, a->status, stream);
+  B200_STEP(gather_scalar, s.dscore, R, a->slots, R, s.grad_route_weights, a->status, stream);
   if (a->grad_w2 != nullptr)
-    B200_STEP(b200moe_grouped_wgrad_bf16(a->rows, D, a->r, F, a->offsets, E, 1, R, D, F, a->grad_w2,
-                                         a->weight_gradients_fp32, a->status, stream));
+    B200_STEP(grouped_wgrad_bf16, a->rows, D, a->r, F, a->offsets, E, 1, R, D, F, a->grad_w2,
+              a->weight_gradients_fp32, a->status, stream);
   if (a->grad_w13 != nullptr) {
-    B200_STEP(b200moe_scatter_rows(a->x, D, T, a->slots, K, R, D, a->rows, D, a->status, stream));
-    B200_STEP(b200moe_grouped_wgrad_bf16(a->gh, 2LL * F, a->rows, D, a->offsets, E, 1, R, 2 * F, D, a->grad_w13,
-                                         a->weight_gradients_fp32, a->status, stream));
+    B200_STEP(scatter_rows, a->x, D, T, a->slots, K, R, D, a->rows, D, a->status, stream);
+    B200_STEP(grouped_wgrad_bf16, a->gh, 2LL * F, a->rows, D, a->offsets, E, 1, R, 2 * F, D, a->grad_w13,
+              a->weight_gradients_fp32, a->status, stream);
   }
-  B200_STEP(b200moe_grouped_gemm_fp8(a->gh_q, 2LL * F, s.gh_scale, 1, R, a->w13, a->w13_scale, a->rows, D, nullptr, 0,
-                                     a->offsets, E, E, R, D, 2 * F, 1, 256, a->status, stream));
-  B200_STEP(b200moe_combine(a->rows, D, R, a->slots, nullptr, nullptr, 0, a->grad_x, D, T, D, K, stream));
+  B200_STEP(grouped_gemm_fp8, a->gh_q, 2LL * F, s.gh_scale, 1, R, a->w13, a->w13_scale, a->rows, D, nullptr, 0,
+            a->offsets, E, E, R, D, 2 * F, 1, 256, a->status, stream);
+  B200_STEP(combine, a->rows, D, R, a->slots, nullptr, nullptr, 0, a->grad_x, D, T, D, K, stream);
   const bool sigmoid = a->mode == B200MOE_ROUTE_SIGMOID_NOAUX_TC;
+  const Range range("b200moe.routing_gradient");
   if (a->grad_aux != nullptr) {
     frequency_kernel<<<(E + 255) / 256, 256, 0, cuda_stream>>>(a->offsets, E, 1.0f / (float)R, sigmoid, s.frequency);
-    B200_STEP(launch_status());
+    const int code = launch_status();
+    if (code != B200MOE_OK) return code;
   }
   return launch_routing_gradient(a->logits, E, T, E, K, a->mode, a->ids, a->route_weights, s.grad_route_weights,
                                  a->grad_aux, a->grad_aux != nullptr ? s.frequency : nullptr,

@@ -55,7 +55,8 @@ class _Timed:
 
 
 # B200MOE_NVTX=1 brackets every wrapper call with an NVTX range named after it, so a timeline
-# shows the phases of a step as the reference's expert-parallel runtime marks its own
+# shows the phases of a step (the library ranges the steps of the one-call layer itself) as the
+# reference's expert-parallel runtime marks its own
 # (src/mlops/expert_parallel/quack/streams.py:36-71). Off by default: a range costs a few
 # hundred nanoseconds on the host per launch.
 NVTX = os.environ.get("B200MOE_NVTX", "0") == "1"
@@ -930,8 +931,8 @@ def dense(t, dtype, *shape):
 
 def whole_layer(x, w13, w2, experts, top_k) -> bool:
     """Whether the one-call forms below serve these operands; the step-by-step form takes the rest
-    (and any call that is being timed or annotated launch by launch)."""
-    if GEMM_TIMINGS is not None or NVTX:
+    (and any call whose GEMMs are being timed launch by launch)."""
+    if GEMM_TIMINGS is not None:
         return False
     (w13_data, w13_scale), (w2_data, w2_scale) = w13, w2
     width, inner = x.shape[1], w2_data.shape[-1]

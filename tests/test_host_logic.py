@@ -126,3 +126,16 @@ def test_ordinary_stores_cross_the_cta_pair_by_release_and_acquire_at_cluster_sc
     assert "if (leader) mbar_arrive(&ready[s]);\n" in report
     assert "else mbar_arrive_remote_release(&ready[s], 0);" in report and "mbar_arrive_remote(" not in report
     assert "mbar_wait_cluster(&ready[s]" in kernel[issuer:] and "mbar_wait(&ready[s]" not in kernel[issuer:]
+
+
+def test_annotated_calls_take_the_path_they_annotate(monkeypatch):
+    """NVTX ranges do not send a call to another form of the layer; timing every GEMM does."""
+    from mlops_b200 import ops
+
+    fp8 = lambda *shape: torch.empty(shape, dtype=torch.float8_e4m3fn)  # noqa: E731
+    x = torch.empty(3, 256, dtype=torch.bfloat16)
+    w13, w2 = (fp8(4, 256, 256), torch.empty(4, 2, 2)), (fp8(4, 256, 128), torch.empty(4, 2, 1))
+    monkeypatch.setattr(ops, "NVTX", True)
+    assert ops.whole_layer(x, w13, w2, 4, 2)
+    monkeypatch.setattr(ops, "GEMM_TIMINGS", [])
+    assert not ops.whole_layer(x, w13, w2, 4, 2)
