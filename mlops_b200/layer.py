@@ -229,8 +229,9 @@ def forward_routed(
 
 def expert_rows(x, order, slots, top_k):
     """bf16 rows of `x [T, D]` in expert order, from the token's side where `slots` is the sort's
-    `[T, K]` (each row is then read once for its copies), else gathered by `order`."""
-    if top_k <= 32 and ops.dense(slots, torch.int32, x.shape[0], top_k):
+    `[T, K]` (each row is then read once for its copies), else gathered by `order`: also where `order` has
+    other than `T * K` rows, which `slots` alone would not give."""
+    if top_k <= 32 and ops.dense(slots, torch.int32, x.shape[0], top_k) and order.numel() == slots.numel():
         return ops.scatter_rows(x, slots)
     return ops.dispatch(x, order, top_k)
 

@@ -139,3 +139,14 @@ def test_annotated_calls_take_the_path_they_annotate(monkeypatch):
     assert ops.whole_layer(x, w13, w2, 4, 2)
     monkeypatch.setattr(ops, "GEMM_TIMINGS", [])
     assert not ops.whole_layer(x, w13, w2, 4, 2)
+
+
+def test_expert_rows_come_from_the_tokens_side_only_where_slots_cover_the_order(monkeypatch):
+    """An `order` of fewer rows, or `slots` of another layout, is gathered row by row as ever."""
+    monkeypatch.setattr(layer.ops, "scatter_rows", lambda x, slots: "scattered")
+    monkeypatch.setattr(layer.ops, "dispatch", lambda x, order, top_k: "gathered")
+    x, slots, order = torch.zeros(3, 8), torch.zeros(3, 2, dtype=torch.int32), torch.zeros(6, dtype=torch.int32)
+    assert layer.expert_rows(x, order, slots, 2) == "scattered"
+    assert layer.expert_rows(x, order[:4], slots, 2) == "gathered"
+    assert layer.expert_rows(x, order, slots.view(6), 2) == "gathered"
+    assert layer.expert_rows(x, order, slots.long(), 2) == "gathered"
